@@ -205,6 +205,8 @@ void fill_desc(const cueva_params* p, const InstGeom& G, int nkslot, double* sla
   };
   I.inv_delx_pow2 = inv_pow2(G.delx);
   I.inv_dely_pow2 = inv_pow2(G.dely);
+  I.recip_delx = 1.0 / G.delx;
+  I.recip_dely = 1.0 / G.dely;
   const double mn = (G.dely < G.delx) ? G.dely : G.delx;   // parameters.f95:329-334
   const double cp = std::sqrt(mn / 1.0);
   I.kappa_psi = 1.0 / (cp * cp);
@@ -1352,6 +1354,8 @@ int32_t cueva_flux_rhs_noalloc(const cueva_params* p, const double* prim, const 
     };
     I.inv_delx_pow2 = inv_pow2(I.delx);
     I.inv_dely_pow2 = inv_pow2(I.dely);
+    I.recip_delx = 1.0 / I.delx;
+    I.recip_dely = 1.0 / I.dely;
   }
   I.c2p = 1;
   I.block_begin[LK_XUPD] = I.block_begin[LK_YFACE] = I.block_begin[LK_STAGE] = 0;

@@ -123,9 +123,9 @@ __global__ void k_fluxandsource(const InstDesc* __restrict__ insts, StageArgs sa
     double qx[NROLE];
 #pragma unroll
     for (int c = 0; c < NROLE; ++c) {
-      const double d = I.fx[c * I.ffs + fo] - I.fx[c * I.ffs + fo - 1];
-      qx[c] = I.inv_delx_pow2 != 0.0 ? d * I.inv_delx_pow2 : d / I.delx;
+      qx[c] = I.fx[c * I.ffs + fo] - I.fx[c * I.ffs + fo - 1];
     }
+    divide_spacing(qx, I.delx, I.inv_delx_pow2, I.recip_delx);
     const double* Q = I.stage[sa.qin];
     const double* pv = I.prim[sa.cur];
     const Centre cv{Q[Q_Q * fs + pc], Q[Q_PSI * fs + pc], Q[Q_PHI * fs + pc], Q[Q_EX * fs + pc],

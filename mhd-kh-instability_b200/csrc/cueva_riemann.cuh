@@ -327,35 +327,33 @@ __device__ __forceinline__ void hllc_fluxes(const Side<T>& L, const Side<T>& R, 
   // star states (:3485-3570)
   const T pstr = Sn_f + (pw2(En_hll) + pw2(Bn_hll)) - (tau_f - ErotB_n) * V;
   const T omV = T(1.0) - V, opV = V + T(1.0);
-  const T psiR = (psi_hll - V * En_f) / omV, psiL = (psi_hll + V * En_f) / opV;
-  const T phiR = (phi_hll - V * Bn_f) / omV, phiL = (phi_hll + V * Bn_f) / opV;
-  const T SnR = (Sn_hll - tau_f * V) / omV, SnL = (Sn_hll + tau_f * V) / opV;
-  const T St1R = (St1_hll - St1_f - ErotB_t1 * V - En_hll * Et1_hll - Bn_hll * Bt1_hll) / omV;
-  const T St1L = (St1_hll + St1_f + ErotB_t1 * V + En_hll * Et1_hll + Bn_hll * Bt1_hll) / opV;
-  const T St2R = (St2_hll - St2_f - ErotB_t2 * V - En_hll * Et2_hll - Bn_hll * Bt2_hll) / omV;
-  const T St2L = (St2_hll + St2_f + ErotB_t2 * V + En_hll * Et2_hll + Bn_hll * Bt2_hll) / opV;
-  const T tauR = (SnR - ErotB_n) / V - pstr + E2B2_str;
-  const T tauL = (SnL - ErotB_n) / V - pstr + E2B2_str;
-  const T DR = (D_hll - D_f) / omV, DL = (D_hll + D_f) / opV;
+  T qR[6] = {psi_hll - V * En_f, phi_hll - V * Bn_f, Sn_hll - tau_f * V,
+             St1_hll - St1_f - ErotB_t1 * V - En_hll * Et1_hll - Bn_hll * Bt1_hll,
+             St2_hll - St2_f - ErotB_t2 * V - En_hll * Et2_hll - Bn_hll * Bt2_hll, D_hll - D_f};
+  T qL[6] = {psi_hll + V * En_f, phi_hll + V * Bn_f, Sn_hll + tau_f * V,
+             St1_hll + St1_f + ErotB_t1 * V + En_hll * Et1_hll + Bn_hll * Bt1_hll,
+             St2_hll + St2_f + ErotB_t2 * V + En_hll * Et2_hll + Bn_hll * Bt2_hll, D_hll + D_f};
+  divide_all(qR, omV, recip_rn(omV));
+  divide_all(qL, opV, recip_rn(opV));
+  const T psiR = qR[0], phiR = qR[1], SnR = qR[2], St1R = qR[3], St2R = qR[4], DR = qR[5];
+  const T psiL = qL[0], phiL = qL[1], SnL = qL[2], St1L = qL[3], St2L = qL[4], DL = qL[5];
+  T qt[2] = {SnR - ErotB_n, SnL - ErotB_n};
+  const T Vd = V == T(0.0) ? T(1.0) : V;   // v* = 0 takes the HLL fluxes: qt is not used
+  divide_all(qt, Vd, recip_rn(Vd));
+  const T tauR = qt[0] - pstr + E2B2_str;
+  const T tauL = qt[1] - pstr + E2B2_str;
   // HLLC flux selection (:3908-4300): s1 < 0 < v* -> left star flux,
   // v* < 0 < s2 -> right star flux, v* == 0 -> HLL flux.  Only psi, phi, D,
   // tau, S receive the star correction; E, B, q keep the HLL fluxes.
-  if (V > T(0.0)) {
-    A[R_PSI] = psi_f + (omV * (psiR - psiL)) * h;
-    A[R_PHI] = phi_f + (omV * (phiR - phiL)) * h;
-    A[R_D] = D_f + omV * (DR - DL) * h;
-    A[R_TAU] = tau_f + omV * (tauR - tauL) * h;
-    A[R_SN] = Sn_f + omV * (SnR - SnL) * h;
-    A[R_ST1] = St1_f + omV * (St1R - St1L) * h;
-    A[R_ST2] = St2_f + omV * (St2R - St2L) * h;
-  } else if (V < T(0.0)) {
-    A[R_PSI] = psi_f + (opV * (psiR - psiL)) * h;
-    A[R_PHI] = phi_f + (opV * (phiR - phiL)) * h;
-    A[R_D] = D_f + opV * (DR - DL) * h;
-    A[R_TAU] = tau_f + opV * (tauR - tauL) * h;
-    A[R_SN] = Sn_f + opV * (SnR - SnL) * h;
-    A[R_ST1] = St1_f + opV * (St1R - St1L) * h;
-    A[R_ST2] = St2_f + opV * (St2R - St2L) * h;
+  if (V > T(0.0) || V < T(0.0)) {
+    const T k = V > T(0.0) ? omV : opV;
+    A[R_PSI] = psi_f + (k * (psiR - psiL)) * h;
+    A[R_PHI] = phi_f + (k * (phiR - phiL)) * h;
+    A[R_D] = D_f + k * (DR - DL) * h;
+    A[R_TAU] = tau_f + k * (tauR - tauL) * h;
+    A[R_SN] = Sn_f + k * (SnR - SnL) * h;
+    A[R_ST1] = St1_f + k * (St1R - St1L) * h;
+    A[R_ST2] = St2_f + k * (St2R - St2L) * h;
   } else if (V == T(0.0)) {
     A[R_D] = D_f; A[R_TAU] = tau_f; A[R_SN] = Sn_f; A[R_ST1] = St1_f; A[R_ST2] = St2_f;
   } else {
@@ -534,34 +532,32 @@ __device__ __forceinline__ void hllcmc_fluxes(const Side<T>& L, const Side<T>& R
   if (vstar) *vstar = V;   // the contact speed the flux choice below uses
   const T pstr = Sn_f + (pw2(En_hll) + pw2(Bn_hll)) - (tau_f - ErotB_n) * V;
   const T omV = T(1.0) - V, opV = V + T(1.0);
-  const T psiR = (psi_hll - V * En_f) / omV, psiL = (psi_hll + V * En_f) / opV;
-  const T phiR = (phi_hll - V * Bn_f) / omV, phiL = (phi_hll + V * Bn_f) / opV;
-  const T SnR = (Sn_hll - tau_f * V) / omV, SnL = (Sn_hll + tau_f * V) / opV;
-  const T St1R = (St1_hll - St1_f - ErotB_t1 * V - En_hll * Et1_hll - Bn_hll * Bt1_hll) / omV;
-  const T St1L = (St1_hll + St1_f + ErotB_t1 * V + En_hll * Et1_hll + Bn_hll * Bt1_hll) / opV;
-  const T St2R = (St2_hll - St2_f - ErotB_t2 * V - En_hll * Et2_hll - Bn_hll * Bt2_hll) / omV;
-  const T St2L = (St2_hll + St2_f + ErotB_t2 * V + En_hll * Et2_hll + Bn_hll * Bt2_hll) / opV;
-  const T tauR = (SnR - ErotB_n) / V - pstr + E2B2_str;
-  const T tauL = (SnL - ErotB_n) / V - pstr + E2B2_str;
-  const T DR = (D_hll - D_f) / omV, DL = (D_hll + D_f) / opV;
+  T qR[6] = {psi_hll - V * En_f, phi_hll - V * Bn_f, Sn_hll - tau_f * V,
+             St1_hll - St1_f - ErotB_t1 * V - En_hll * Et1_hll - Bn_hll * Bt1_hll,
+             St2_hll - St2_f - ErotB_t2 * V - En_hll * Et2_hll - Bn_hll * Bt2_hll, D_hll - D_f};
+  T qL[6] = {psi_hll + V * En_f, phi_hll + V * Bn_f, Sn_hll + tau_f * V,
+             St1_hll + St1_f + ErotB_t1 * V + En_hll * Et1_hll + Bn_hll * Bt1_hll,
+             St2_hll + St2_f + ErotB_t2 * V + En_hll * Et2_hll + Bn_hll * Bt2_hll, D_hll + D_f};
+  divide_all(qR, omV, recip_rn(omV));
+  divide_all(qL, opV, recip_rn(opV));
+  const T psiR = qR[0], phiR = qR[1], SnR = qR[2], St1R = qR[3], St2R = qR[4], DR = qR[5];
+  const T psiL = qL[0], phiL = qL[1], SnL = qL[2], St1L = qL[3], St2L = qL[4], DL = qL[5];
+  T qt[2] = {SnR - ErotB_n, SnL - ErotB_n};
+  const T Vd = V == T(0.0) ? T(1.0) : V;   // v* = 0 takes the HLL fluxes: qt is not used
+  divide_all(qt, Vd, recip_rn(Vd));
+  const T tauR = qt[0] - pstr + E2B2_str;
+  const T tauL = qt[1] - pstr + E2B2_str;
   // flux choice (:3530-3620): v* > 0 left star flux, v* < 0 right star flux,
   // v* == 0 the HLL fluxes; E, B and q keep the HLL fluxes throughout
-  if (V > T(0.0)) {
-    A[R_PSI] = psi_f + (omV * (psiR - psiL)) * h;
-    A[R_PHI] = phi_f + (omV * (phiR - phiL)) * h;
-    A[R_D] = D_f + omV * (DR - DL) * h;
-    A[R_TAU] = tau_f + omV * (tauR - tauL) * h;
-    A[R_SN] = Sn_f + omV * (SnR - SnL) * h;
-    A[R_ST1] = St1_f + omV * (St1R - St1L) * h;
-    A[R_ST2] = St2_f + omV * (St2R - St2L) * h;
-  } else if (V < T(0.0)) {
-    A[R_PSI] = psi_f + (opV * (psiR - psiL)) * h;
-    A[R_PHI] = phi_f + (opV * (phiR - phiL)) * h;
-    A[R_D] = D_f + opV * (DR - DL) * h;
-    A[R_TAU] = tau_f + opV * (tauR - tauL) * h;
-    A[R_SN] = Sn_f + opV * (SnR - SnL) * h;
-    A[R_ST1] = St1_f + opV * (St1R - St1L) * h;
-    A[R_ST2] = St2_f + opV * (St2R - St2L) * h;
+  if (V > T(0.0) || V < T(0.0)) {
+    const T k = V > T(0.0) ? omV : opV;
+    A[R_PSI] = psi_f + (k * (psiR - psiL)) * h;
+    A[R_PHI] = phi_f + (k * (phiR - phiL)) * h;
+    A[R_D] = D_f + k * (DR - DL) * h;
+    A[R_TAU] = tau_f + k * (tauR - tauL) * h;
+    A[R_SN] = Sn_f + k * (SnR - SnL) * h;
+    A[R_ST1] = St1_f + k * (St1R - St1L) * h;
+    A[R_ST2] = St2_f + k * (St2R - St2L) * h;
   } else if (!(V == T(0.0))) {
     st |= ST_HLLC_VSTAR;
 #pragma unroll

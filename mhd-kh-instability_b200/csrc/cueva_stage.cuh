@@ -690,11 +690,11 @@ __device__ __forceinline__ uint32_t update_point(const InstDesc& I, const StageA
   const double* __restrict__ aux = I.aux[sa.cur];
   uint32_t st = 0;
   const long long pc = (long long)j * pitch + i;
-  const double dly = I.dely, iy2 = I.inv_dely_pow2;
-  auto qy = [&](int r) {   // (dy)/dly
-    const double d = fyd(r);
-    return iy2 != 0.0 ? d * iy2 : d / dly;
-  };
+  double dy[NROLE];   // (dy)/dely
+#pragma unroll
+  for (int c = 0; c < NROLE; ++c) dy[c] = fyd(c);
+  divide_spacing(dy, I.dely, I.inv_dely_pow2, I.recip_dely);
+  auto qy = [&](int r) { return dy[r]; };
   auto qxf = [&](int r) { return qx[r]; };
   const double q = cv.q, psi = cv.psi, phi = cv.phi, Ex = cv.Ex, Ey = cv.Ey, Ez = cv.Ez;
   const double Bx = cv.Bx, By = cv.By, Bz = cv.Bz, vx = cv.vx, vy = cv.vy, vz = cv.vz;
@@ -749,6 +749,7 @@ __device__ __forceinline__ uint32_t update_point(const InstDesc& I, const StageA
       double acc[NCONS];
 #pragma unroll
       for (int c = 0; c < NCONS; ++c) acc[c] = sa.need_intsum_load ? I.intsum[c * fs + pc] : 0.0;
+#pragma unroll 1
       for (int m = 1; m <= sa.l; ++m) {
         const double ab = sa.ab_next[m - 1], abt = sa.abt_next[m - 1];
         if (ab == 0.0 && abt == 0.0) continue;
@@ -915,15 +916,13 @@ __device__ __forceinline__ void xupd_tile(const InstDesc& I, const StageArgs& sa
     }
   }
   // Fx(i-1/2) of point i is the face of lane-1
-  const double dlx = I.delx, ix2 = I.inv_delx_pow2;
   double qx[NROLE];
 #pragma unroll
   for (int c = 0; c < NROLE; ++c) {
     const double fr = double(F[c]);
-    const double fl = __shfl_up_sync(0xffffffffu, fr, 1);
-    const double d = fr - fl;
-    qx[c] = ix2 != 0.0 ? d * ix2 : d / dlx;
+    qx[c] = fr - __shfl_up_sync(0xffffffffu, fr, 1);
   }
+  divide_spacing(qx, I.delx, I.inv_delx_pow2, I.recip_delx);
   const bool valid = lane >= 1 && i <= ilast;
   // after the last stage every lane of the warp enters the update (lanes
   // without a point repeat a real one and store nothing), so con2prim runs
@@ -1334,15 +1333,13 @@ k_stage(const InstDesc* __restrict__ insts, int ninst, int ntiles, StageArgs sa)
         ring_fill<RM, ROWS>(I, sa, ring, i0, ilast, j0 + ROWS + R + 1, min(j0 + 2 * ROWS - 1, jend) + R + 1, tid,
                             bulk, &bar);
       if (j <= jl && !face_only) {
-        const double dlx = I.delx, ix2 = I.inv_delx_pow2;
         double qx[NROLE];
 #pragma unroll
         for (int c = 0; c < NROLE; ++c) {
           const double fr = double(Fx[c]);
-          const double fl = __shfl_up_sync(0xffffffffu, fr, 1);
-          const double d = fr - fl;
-          qx[c] = ix2 != 0.0 ? d * ix2 : d / dlx;
+          qx[c] = fr - __shfl_up_sync(0xffffffffu, fr, 1);
         }
+        divide_spacing(qx, I.delx, I.inv_delx_pow2, I.recip_delx);
         if (valid || warp_c2p) {
           if (warp_c2p) {
 #pragma unroll
