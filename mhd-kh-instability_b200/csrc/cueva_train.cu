@@ -2,15 +2,16 @@
 // seed (cueva_mlp.cuh), on the GPU with this file's own kernels:
 //   * synthetic (conserved, primitive) pairs from a counter-based generator;
 //   * feature extraction and normalisation statistics;
-//   * minibatch SGD with Adam: forward and backward passes as small tiled
-//     FP32 GEMMs over bf16-rounded weights (the same rounding the inference
-//     kernels read), SiLU and its derivative, bias sums, loss;
+//   * minibatch SGD with Adam: the forward and backward pass of a batch in one
+//     kernel (FP32 over bf16-rounded weights, the same rounding the inference
+//     kernels read), and one that sums the CTAs' gradients and applies Adam;
 //   * batch con2prim for the ablation: Cardano, network seed + Newton, or a
 //     given seed + Newton, with the Newton iteration count per state.
 // The C-ABI entry points are declared in include/cueva.h.
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -118,105 +119,289 @@ __global__ void k_moments(long long n, const float* X, const float* T, double* a
   }
 }
 
-// minibatch rows (uniform with replacement; all rows when seed == 0) with
-// the normalisation applied
-__global__ void k_gather(long long n, int B, unsigned long long seed, long long step, const float* X, const float* T,
-                         const float* norm, float* Xb, float* Tb) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= B) return;
-  const long long row = seed ? (long long)(mix64(seed ^ mix64((unsigned long long)step * 1048576ull + b)) % (unsigned long long)n)
-                             : (long long)b;
+// One training batch, forward and backward, in one launch.
+//
+// A CTA takes tiles of 32 rows: features (from the stored ones, or from the
+// states themselves), the three hidden layers, the loss and the backward
+// pass, with the weights (bf16-rounded, transposed) and every activation of
+// the tile in shared memory; its share of the weight gradients stays in
+// registers over its tiles and goes to one row of `part`, which
+// k_reduce_gradients sums in a fixed order (deterministic).
+//
+// The passes of a 4096-row batch are 0.1 GFMA: what counts is the number of
+// dependent launches and the length of the serial sums, not the arithmetic.
+// As 24 launches of small GEMMs, with the weight gradients as one 4096-long
+// sum per output on 16 CTAs, a gradient call took 598 us (B200; 170 us in
+// each of the four weight-gradient GEMMs).  Split over 128 CTAs of 32 rows the
+// longest sum is 32 rows and then 128 partial sums; see k_reduce_gradients
+// for the times.  Forward values, dY, dZ and dA keep the order of operations
+// of single dot products (ascending index, one FMA each).
+constexpr int GT_ROWS = 32;          // rows of a tile
+constexpr int GT_THREADS = 256;
+constexpr int GT_LD = 68;            // activation row stride: float4 rows, banks shifted by 4
+constexpr int GT_LW = MLP_H + 1;     // transposed weight row stride: conflict-free both ways
+constexpr int GT_PART = (MLP_NPARAM + 1 + 31) / 32 * 32;   // a partial row: gradients, then the loss sum
+
+struct GradTile {
+  float w1t[MLP_IN * GT_LW], w2t[MLP_H * GT_LW], w3t[MLP_H * GT_LW], w4[MLP_H];
+  float b1[MLP_H], b2[MLP_H], b3[MLP_H], b4;
+  float x[GT_ROWS * 8];              // normalised features
+  float t[GT_ROWS], dy[GT_ROWS], d2[GT_ROWS];
+  alignas(16) float z1[GT_ROWS * GT_LD], a1[GT_ROWS * GT_LD], z2[GT_ROWS * GT_LD], a2[GT_ROWS * GT_LD],
+      z3[GT_ROWS * GT_LD], a3[GT_ROWS * GT_LD], dz[GT_ROWS * GT_LD];
+};
+
+// rows 4 w .. 4 w + 3 of C = A B (K = 64) for warp w, lane l holding columns
+// l and l + 32: acc[r][c] over ascending k; B(k, n) = bt[k * sk + n * sn]
+__device__ __forceinline__ void tile_dot(const float* a, const float* bt, int sk, int sn, float (&acc)[4][2]) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const float* b0 = bt + lane * sn;
+  const float* b1 = bt + (lane + 32) * sn;
 #pragma unroll
-  for (int k = 0; k < MLP_IN; ++k) Xb[b * MLP_IN + k] = (X[row * MLP_IN + k] - norm[k]) / norm[MLP_IN + k];
-  Tb[b] = (T[row] - norm[2 * MLP_IN]) / norm[2 * MLP_IN + 1];
+  for (int r = 0; r < 4; ++r) acc[r][0] = acc[r][1] = 0.0f;
+#pragma unroll 4
+  for (int k = 0; k < MLP_H; k += 4) {
+    float4 av[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) av[r] = *reinterpret_cast<const float4*>(a + (4 * w + r) * GT_LD + k);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float u = b0[(k + q) * sk], v = b1[(k + q) * sk];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const float x = q == 0 ? av[r].x : q == 1 ? av[r].y : q == 2 ? av[r].z : av[r].w;
+        acc[r][0] = fmaf(x, u, acc[r][0]);
+        acc[r][1] = fmaf(x, v, acc[r][1]);
+      }
+    }
+  }
+}
+__device__ __forceinline__ float silu_slope(float z) {
+  const float s = sigmoid_fast(z);
+  return s * (1.0f + z * (1.0f - s));
+}
+// hidden layer: z = a W^T + b, act = silu(z)
+__device__ __forceinline__ void tile_layer(const float* a, const float* wt, const float* b, float* z, float* act) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  float acc[4][2];
+  tile_dot(a, wt, GT_LW, 1, acc);
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const int o = lane + 32 * c, e = (4 * w + r) * GT_LD + o;
+      const float v = acc[r][c] + b[o];
+      z[e] = v;
+      act[e] = silu(v);
+    }
+}
+// dz of the layer below, in place: dz <- (dz W) silu'(z); every warp reads
+// and writes its own four rows
+__device__ __forceinline__ void tile_back(float* dz, const float* wt, const float* z) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  float acc[4][2];
+  tile_dot(dz, wt, 1, GT_LW, acc);   // B(o, i) = W(o, i) = wt[i][o]
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const int e = (4 * w + r) * GT_LD + lane + 32 * c;
+      dz[e] = acc[r][c] * silu_slope(z[e]);
+    }
+}
+// dw[a][b] += sum over the tile's rows of dz(row, to + 16 a) act(row, ti + 16 b)
+__device__ __forceinline__ void tile_outer(const float* dz, const float* act, float (&dw)[4][4]) {
+  const int ti = threadIdx.x & 15, to = threadIdx.x >> 4;
+#pragma unroll 4
+  for (int r = 0; r < GT_ROWS; ++r) {
+    float u[4], v[4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) { u[a] = dz[r * GT_LD + to + 16 * a]; v[a] = act[r * GT_LD + ti + 16 * a]; }
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) dw[a][b] = fmaf(u[a], v[b], dw[a][b]);
+  }
 }
 
-// C[m][n] (+)= sum_k A(m,k) B(k,n); A(m,k) = TA ? A[k*lda+m] : A[m*lda+k],
-// B(k,n) = TB ? B[n*ldb+k] : B[k*ldb+n]; bias[n] added when non-null;
-// with SILU the pre-activation goes to Z and silu(Z) to C.
-template <bool TA, bool TB, bool SILU>
-__global__ void __launch_bounds__(256) k_gemm(int M, int N, int K, const float* __restrict__ A, int lda,
-                                              const float* __restrict__ Bm, int ldb, const float* __restrict__ bias,
-                                              float* __restrict__ C, int ldc, float* __restrict__ Z) {
-  __shared__ float sa[16][17], sb[16][17];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int m = blockIdx.y * 16 + ty, nn = blockIdx.x * 16 + tx;
-  float acc = 0.0f;
-  for (int k0 = 0; k0 < K; k0 += 16) {
-    {
-      const int mm = blockIdx.y * 16 + ty, kk = k0 + tx;
-      sa[ty][tx] = (mm < M && kk < K) ? (TA ? A[(long long)kk * lda + mm] : A[(long long)mm * lda + kk]) : 0.0f;
-      const int kb = k0 + ty, nb = blockIdx.x * 16 + tx;
-      sb[ty][tx] = (kb < K && nb < N) ? (TB ? Bm[(long long)nb * ldb + kb] : Bm[(long long)kb * ldb + nb]) : 0.0f;
+// B rows: row b itself (seed == 0), or drawn uniformly with replacement from
+// n.  X, T: stored raw features and targets; with X null they are computed
+// from the states (cons, p).
+__global__ void __launch_bounds__(GT_THREADS)
+k_gradients(long long n, int B, unsigned long long seed, long long step, const float* __restrict__ X,
+            const float* __restrict__ T, const double* __restrict__ cons, const double* __restrict__ p,
+            const float* __restrict__ norm, const float* __restrict__ wr, float* __restrict__ part) {
+  extern __shared__ __align__(16) unsigned char gt_smem[];
+  GradTile& S = *reinterpret_cast<GradTile*>(gt_smem);
+  const int tid = threadIdx.x;
+  for (int e = tid; e < MLP_H * MLP_IN; e += GT_THREADS)
+    S.w1t[(e % MLP_IN) * GT_LW + e / MLP_IN] = wr[MLP_OFF_W1 + e];
+  for (int e = tid; e < MLP_H * MLP_H; e += GT_THREADS) {
+    S.w2t[(e % MLP_H) * GT_LW + e / MLP_H] = wr[MLP_OFF_W2 + e];
+    S.w3t[(e % MLP_H) * GT_LW + e / MLP_H] = wr[MLP_OFF_W3 + e];
+  }
+  if (tid < MLP_H) {
+    S.w4[tid] = wr[MLP_OFF_W4 + tid];
+    S.b1[tid] = wr[MLP_OFF_B1 + tid];
+    S.b2[tid] = wr[MLP_OFF_B2 + tid];
+    S.b3[tid] = wr[MLP_OFF_B3 + tid];
+    if (tid == 0) S.b4 = wr[MLP_OFF_B4];
+  }
+  float g3[4][4] = {}, g2[4][4] = {};   // W3, W2: outputs to + 16 a, inputs ti + 16 b
+  float g1[2] = {}, gb = 0.0f, gl = 0.0f;   // W1 elements tid, tid + 256; a bias or W4 element; b4 or the loss
+  for (long long r0 = (long long)blockIdx.x * GT_ROWS; r0 < B; r0 += (long long)gridDim.x * GT_ROWS) {
+    __syncthreads();   // the tile before has been read
+    if (tid < GT_ROWS) {
+      const long long b = r0 + tid;
+      float f[MLP_IN] = {}, t = 0.0f;
+      if (b < B) {
+        const long long row =
+            seed ? (long long)(mix64(seed ^ mix64((unsigned long long)step * 1048576ull + b)) % (unsigned long long)n)
+                 : b;
+        if (X) {
+#pragma unroll
+          for (int k = 0; k < MLP_IN; ++k) f[k] = X[row * MLP_IN + k];
+          t = T[row];
+        } else {
+          c2p_features(cons[row], cons[n + row], cons[2 * n + row], cons[3 * n + row], cons[4 * n + row],
+                       cons[5 * n + row], cons[6 * n + row], cons[7 * n + row], cons[8 * n + row], cons[9 * n + row],
+                       cons[10 * n + row], f);
+          t = (float)log(p[row] / cons[row]);
+        }
+#pragma unroll
+        for (int k = 0; k < MLP_IN; ++k) f[k] = (f[k] - norm[k]) / norm[MLP_IN + k];
+        t = (t - norm[2 * MLP_IN]) / norm[2 * MLP_IN + 1];
+      }
+#pragma unroll
+      for (int k = 0; k < MLP_IN; ++k) S.x[tid * 8 + k] = f[k];
+      S.t[tid] = t;
     }
     __syncthreads();
+    {   // first layer (K = 6)
+      const int lane = tid & 31, w = tid >> 5;
 #pragma unroll
-    for (int k = 0; k < 16; ++k) acc = fmaf(sa[ty][k], sb[k][tx], acc);
-    __syncthreads();
-  }
-  if (m < M && nn < N) {
-    if (bias) acc += bias[nn];
-    if (SILU) {
-      Z[(long long)m * ldc + nn] = acc;
-      acc = silu(acc);
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int o = lane + 32 * c, row = 4 * w + r;
+          float v = 0.0f;
+#pragma unroll
+          for (int k = 0; k < MLP_IN; ++k) v = fmaf(S.x[row * 8 + k], S.w1t[k * GT_LW + o], v);
+          v += S.b1[o];
+          S.z1[row * GT_LD + o] = v;
+          S.a1[row * GT_LD + o] = silu(v);
+        }
     }
-    C[(long long)m * ldc + nn] = acc;
-  }
-}
-
-// loss = mean (y - t)^2 over the batch, dY = 2 (y - t) / B
-__global__ void k_loss(int B, const float* Y, const float* T, float* dY, float* loss) {
-  float s = 0.0f;
-  for (int b = threadIdx.x; b < B; b += blockDim.x) {
-    const float d = Y[b] - T[b];
-    dY[b] = 2.0f * d / (float)B;
-    s += d * d;
-  }
-  __shared__ float red[256];
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+    __syncwarp();   // a warp reads its own four rows only
+    tile_layer(S.a1, S.w2t, S.b2, S.z2, S.a2);
+    __syncwarp();
+    tile_layer(S.a2, S.w3t, S.b3, S.z3, S.a3);
     __syncthreads();
-  }
-  if (threadIdx.x == 0) *loss = red[0] / (float)B;
-}
-
-// dZ = dA * silu'(Z)
-__global__ void k_silu_back(long long n, const float* dA, const float* Z, float* dZ) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const float z = Z[i], s = sigmoid_fast(z);
-    dZ[i] = dA[i] * (s * (1.0f + z * (1.0f - s)));
-  }
-}
-
-// db[n] = sum_b dZ[b][n]
-__global__ void k_colsum(int B, int N, const float* dZ, float* db) {
-  const int nn = blockIdx.x;
-  float s = 0.0f;
-  for (int b = threadIdx.x; b < B; b += blockDim.x) s += dZ[(long long)b * N + nn];
-  __shared__ float red[256];
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+    if (tid < GT_ROWS) {   // output, loss and its gradient (rows past the batch count nothing)
+      float y = 0.0f;
+#pragma unroll 8
+      for (int k = 0; k < MLP_H; ++k) y = fmaf(S.a3[tid * GT_LD + k], S.w4[k], y);
+      y += S.b4;
+      const float d = r0 + tid < B ? y - S.t[tid] : 0.0f;
+      S.dy[tid] = 2.0f * d / (float)B;
+      S.d2[tid] = d * d;
+    }
     __syncthreads();
+    {   // dZ3 = dY W4 silu'(Z3)
+      const int lane = tid & 31, w = tid >> 5;
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int o = lane + 32 * c, e = (4 * w + r) * GT_LD + o;
+          S.dz[e] = (S.dy[4 * w + r] * S.w4[o]) * silu_slope(S.z3[e]);
+        }
+    }
+    __syncthreads();
+    // column sums by groups of 64 threads: b3 (dZ3) here, W4 (dY A3), later b2 and b1
+    const int col = tid & 63, grp = tid >> 6;
+    if (grp == 0) {
+      for (int r = 0; r < GT_ROWS; ++r) gb += S.dz[r * GT_LD + col];
+    } else if (grp == 3) {
+      for (int r = 0; r < GT_ROWS; ++r) gb = fmaf(S.dy[r], S.a3[r * GT_LD + col], gb);
+    }
+    if (tid == 64)
+      for (int r = 0; r < GT_ROWS; ++r) gl += S.dy[r];
+    if (tid == 128)
+      for (int r = 0; r < GT_ROWS; ++r) gl += S.d2[r];
+    tile_outer(S.dz, S.a2, g3);
+    __syncthreads();
+    tile_back(S.dz, S.w3t, S.z2);
+    __syncthreads();
+    if (grp == 1)
+      for (int r = 0; r < GT_ROWS; ++r) gb += S.dz[r * GT_LD + col];
+    tile_outer(S.dz, S.a1, g2);
+    __syncthreads();
+    tile_back(S.dz, S.w2t, S.z1);
+    __syncthreads();
+    if (grp == 2)
+      for (int r = 0; r < GT_ROWS; ++r) gb += S.dz[r * GT_LD + col];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int e = tid + 256 * q, o = e / MLP_IN, k = e % MLP_IN;
+      if (e < MLP_H * MLP_IN)
+        for (int r = 0; r < GT_ROWS; ++r) g1[q] = fmaf(S.dz[r * GT_LD + o], S.x[r * 8 + k], g1[q]);
+    }
   }
-  if (threadIdx.x == 0) db[nn] = red[0];
+  float* out = part + (long long)blockIdx.x * GT_PART;
+  const int ti = tid & 15, to = tid >> 4;
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      out[MLP_OFF_W3 + (to + 16 * a) * MLP_H + ti + 16 * b] = g3[a][b];
+      out[MLP_OFF_W2 + (to + 16 * a) * MLP_H + ti + 16 * b] = g2[a][b];
+    }
+#pragma unroll
+  for (int q = 0; q < 2; ++q)
+    if (tid + 256 * q < MLP_H * MLP_IN) out[MLP_OFF_W1 + tid + 256 * q] = g1[q];
+  const int col = tid & 63, grp = tid >> 6;
+  out[(grp == 0 ? MLP_OFF_B3 : grp == 1 ? MLP_OFF_B2 : grp == 2 ? MLP_OFF_B1 : MLP_OFF_W4) + col] = gb;
+  if (tid == 64) out[MLP_OFF_B4] = gl;
+  if (tid == 128) out[MLP_NPARAM] = gl;
 }
 
-// Adam (Kingma & Ba 2015) and the bf16 rounding of the forward copy
-__global__ void k_adam(int n, float* w, float* m, float* v, const float* g, float* wr, float lr, float b1, float b2,
-                       float c1, float c2) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float gi = g[i];
-  const float mi = b1 * m[i] + (1.0f - b1) * gi;
-  const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-  m[i] = mi; v[i] = vi;
-  const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + 1.0e-8f);
-  w[i] = wi;
-  wr[i] = __bfloat162float(__float2bfloat16(wi));
+// Sums the nrows partial rows of k_gradients into g (and the loss / B behind
+// it) and, with ADAM, applies the update (Kingma & Ba 2015) and the bf16
+// rounding of the forward copy.  A CTA takes 32 parameters by 8 slices of the
+// rows, each slice in order, the 8 slice sums in order.  B200, 4096 rows,
+// whole gradient call: 600 us before, 57 us with these two kernels (25 + 4 us
+// under ncu, the rest is the copy back); 2000 training steps 1.09 s -> 50 ms.
+template <bool ADAM>
+__global__ void __launch_bounds__(256)
+k_reduce_gradients(int nrows, const float* __restrict__ part, float* g, int B, float* w, float* m, float* v, float* wr,
+                   float lr, float b1, float b2, float c1, float c2) {
+  __shared__ float sum[8][32];
+  const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5;
+  const int i = blockIdx.x * 32 + lane;   // GT_PART is a multiple of 32
+  float s = 0.0f;
+#pragma unroll 8
+  for (int r = sl; r < nrows; r += 8) s += part[(long long)r * GT_PART + i];
+  sum[sl][lane] = s;
+  __syncthreads();
+  if (sl != 0 || i > MLP_NPARAM) return;
+  float gi = sum[0][lane];
+#pragma unroll
+  for (int k = 1; k < 8; ++k) gi += sum[k][lane];
+  if (i == MLP_NPARAM) {
+    g[i] = gi / (float)B;   // the loss
+    return;
+  }
+  g[i] = gi;
+  if constexpr (ADAM) {
+    const float mi = b1 * m[i] + (1.0f - b1) * gi;
+    const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
+    m[i] = mi; v[i] = vi;
+    const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + 1.0e-8f);
+    w[i] = wi;
+    wr[i] = __bfloat162float(__float2bfloat16(wi));
+  }
 }
 
 __global__ void k_round(int n, const float* w, float* wr) {
@@ -277,76 +462,34 @@ dim3 grid_for(long long n) {
 // ---------------------------------------------------------------- the object
 struct cueva_mlp {
   int dev = 0;
-  int bmax = 0;
   float* w = nullptr;      // FP32 master parameters
   float* wr = nullptr;     // bf16-rounded copy read by the forward passes
   float* m = nullptr;
   float* v = nullptr;
-  float* g = nullptr;
+  float* g = nullptr;      // gradients, then the loss
   float* norm = nullptr;   // device copy of hnorm
   float hnorm[MLP_NNORM];
   bool normed = false;
   long long step = 0;
-  // batch work space
-  float *Xb = nullptr, *Tb = nullptr, *Z1 = nullptr, *A1 = nullptr, *Z2 = nullptr, *A2 = nullptr, *Z3 = nullptr,
-        *A3 = nullptr, *Y = nullptr, *dY = nullptr, *dA = nullptr, *dZ = nullptr, *loss = nullptr;
+  float* part = nullptr;   // partial gradients of k_gradients: GT_GRID rows
   MLPDevice* d_dev = nullptr;
 };
 
 namespace {
 
-void free_batch(cueva_mlp* M) {
-  for (float** p : {&M->Xb, &M->Tb, &M->Z1, &M->A1, &M->Z2, &M->A2, &M->Z3, &M->A3, &M->Y, &M->dY, &M->dA, &M->dZ})
-    if (*p) { cudaFree(*p); *p = nullptr; }
-  M->bmax = 0;
-}
+// CTAs of k_gradients: a tile each, at most two per SM of a B200
+constexpr int GT_GRID = 2 * 148;
+int gradient_grid(int B) { return std::min((B - 1) / GT_ROWS + 1, GT_GRID); }
 
-int32_t ensure_batch(cueva_mlp* M, int B) {
-  if (B <= M->bmax) return CUEVA_OK;
-  free_batch(M);
-  const size_t h = (size_t)B * MLP_H * sizeof(float);
-  TRY(cudaMalloc(&M->Xb, (size_t)B * MLP_IN * sizeof(float)));
-  TRY(cudaMalloc(&M->Tb, (size_t)B * sizeof(float)));
-  for (float** p : {&M->Z1, &M->A1, &M->Z2, &M->A2, &M->Z3, &M->A3, &M->dA, &M->dZ}) TRY(cudaMalloc(p, h));
-  TRY(cudaMalloc(&M->Y, (size_t)B * sizeof(float)));
-  TRY(cudaMalloc(&M->dY, (size_t)B * sizeof(float)));
-  M->bmax = B;
-  return CUEVA_OK;
-}
-
-template <bool TA, bool TB, bool SILU>
-void gemm(int Mr, int N, int K, const float* A, int lda, const float* B, int ldb, const float* bias, float* C,
-          int ldc, float* Z = nullptr) {
-  const dim3 grid((N + 15) / 16, (Mr + 15) / 16);
-  k_gemm<TA, TB, SILU><<<grid, 256>>>(Mr, N, K, A, lda, B, ldb, bias, C, ldc, Z);
-}
-
-// forward and backward of one batch already gathered in Xb/Tb; gradients in g
-int32_t forward_backward(cueva_mlp* M, int B) {
-  const float* W = M->wr;
-  float* G = M->g;
-  const int H = MLP_H;
-  // forward: Z = X W^T + b, A = silu(Z)
-  gemm<false, true, true>(B, H, MLP_IN, M->Xb, MLP_IN, W + MLP_OFF_W1, MLP_IN, W + MLP_OFF_B1, M->A1, H, M->Z1);
-  gemm<false, true, true>(B, H, H, M->A1, H, W + MLP_OFF_W2, H, W + MLP_OFF_B2, M->A2, H, M->Z2);
-  gemm<false, true, true>(B, H, H, M->A2, H, W + MLP_OFF_W3, H, W + MLP_OFF_B3, M->A3, H, M->Z3);
-  gemm<false, true, false>(B, 1, H, M->A3, H, W + MLP_OFF_W4, H, W + MLP_OFF_B4, M->Y, 1);
-  k_loss<<<1, 256>>>(B, M->Y, M->Tb, M->dY, M->loss);
-  // backward
-  gemm<true, false, false>(1, H, B, M->dY, 1, M->A3, H, nullptr, G + MLP_OFF_W4, H);         // dW4 = dY^T A3
-  k_colsum<<<1, 256>>>(B, 1, M->dY, G + MLP_OFF_B4);
-  gemm<false, false, false>(B, H, 1, M->dY, 1, W + MLP_OFF_W4, H, nullptr, M->dA, H);        // dA3 = dY W4
-  k_silu_back<<<grid_for((long long)B * H), 256>>>((long long)B * H, M->dA, M->Z3, M->dZ);
-  gemm<true, false, false>(H, H, B, M->dZ, H, M->A2, H, nullptr, G + MLP_OFF_W3, H);         // dW3 = dZ3^T A2
-  k_colsum<<<H, 256>>>(B, H, M->dZ, G + MLP_OFF_B3);
-  gemm<false, false, false>(B, H, H, M->dZ, H, W + MLP_OFF_W3, H, nullptr, M->dA, H);        // dA2 = dZ3 W3
-  k_silu_back<<<grid_for((long long)B * H), 256>>>((long long)B * H, M->dA, M->Z2, M->dZ);
-  gemm<true, false, false>(H, H, B, M->dZ, H, M->A1, H, nullptr, G + MLP_OFF_W2, H);         // dW2 = dZ2^T A1
-  k_colsum<<<H, 256>>>(B, H, M->dZ, G + MLP_OFF_B2);
-  gemm<false, false, false>(B, H, H, M->dZ, H, W + MLP_OFF_W2, H, nullptr, M->dA, H);        // dA1 = dZ2 W2
-  k_silu_back<<<grid_for((long long)B * H), 256>>>((long long)B * H, M->dA, M->Z1, M->dZ);
-  gemm<true, false, false>(H, MLP_IN, B, M->dZ, H, M->Xb, MLP_IN, nullptr, G + MLP_OFF_W1, MLP_IN);  // dW1
-  k_colsum<<<H, 256>>>(B, H, M->dZ, G + MLP_OFF_B1);
+// launches the passes of one batch; the partial gradients go to M->part
+int32_t forward_backward(cueva_mlp* M, long long n, int B, unsigned long long seed, const float* X, const float* T,
+                         const double* cons, const double* p) {
+  if (!M->part) {
+    TRY(cudaFuncSetAttribute(k_gradients, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GradTile)));
+    TRY(cudaMalloc(&M->part, (size_t)GT_GRID * GT_PART * sizeof(float)));
+  }
+  k_gradients<<<gradient_grid(B), GT_THREADS, sizeof(GradTile)>>>(n, B, seed, M->step, X, T, cons, p, M->norm, M->wr,
+                                                                  M->part);
   TRY(cudaGetLastError());
   return CUEVA_OK;
 }
@@ -425,9 +568,8 @@ int32_t cueva_mlp_create(int32_t device, uint64_t seed, cueva_mlp** out) {
   for (int k = 0; k < MLP_NNORM; ++k) M->hnorm[k] = (k >= MLP_IN && k < 2 * MLP_IN) || k == 2 * MLP_IN + 1 ? 1.0f : 0.0f;
   cudaError_t e = cudaSuccess;
   for (float** p : {&M->w, &M->wr, &M->m, &M->v, &M->g})
-    if (e == cudaSuccess) e = cudaMalloc(p, MLP_NPARAM * sizeof(float));
+    if (e == cudaSuccess) e = cudaMalloc(p, (MLP_NPARAM + 1) * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc(&M->norm, MLP_NNORM * sizeof(float));
-  if (e == cudaSuccess) e = cudaMalloc(&M->loss, sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc(&M->d_dev, sizeof(MLPDevice));
   if (e == cudaSuccess) e = cudaMemcpy(M->w, w.data(), MLP_NPARAM * sizeof(float), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemset(M->m, 0, MLP_NPARAM * sizeof(float));
@@ -449,8 +591,7 @@ int32_t cueva_mlp_destroy(cueva_mlp* M) {
   if (!M) return CUEVA_OK;
   cudaSetDevice(M->dev);
   cudaDeviceSynchronize();
-  free_batch(M);
-  for (float* p : {M->w, M->wr, M->m, M->v, M->g, M->norm, M->loss})
+  for (float* p : {M->w, M->wr, M->m, M->v, M->g, M->norm, M->part})
     if (p) cudaFree(p);
   if (M->d_dev) cudaFree(M->d_dev);
   delete M;
@@ -528,24 +669,23 @@ int32_t cueva_mlp_train(cueva_mlp* M, const double* d_cons, const double* d_p, i
   if (!M || n <= 0 || steps < 0 || batch <= 0 || !d_cons || !d_p) return cueva_fail(CUEVA_ERR_ARG, "bad arguments");
   if (!M->normed) return cueva_fail(CUEVA_ERR_ARG, "fit the normalisation first");
   TRY(cudaSetDevice(M->dev));
-  if (int32_t e = ensure_batch(M, batch)) return e;
   float *X = nullptr, *T = nullptr;
   int32_t rc = features_of(n, d_cons, d_p, &X, &T);
   const float b1 = 0.9f, b2 = 0.999f;
   for (int s = 0; s < steps && !rc; ++s) {
     ++M->step;
-    k_gather<<<(batch + 255) / 256, 256>>>(n, batch, seed ? seed : 1ull, M->step, X, T, M->norm, M->Xb, M->Tb);
-    rc = forward_backward(M, batch);
+    rc = forward_backward(M, n, batch, seed ? seed : 1ull, X, T, nullptr, nullptr);
     if (rc) break;
     // cosine decay of the learning rate over this call's steps
     const float lr_s = 0.5f * lr * (1.0f + std::cos(3.14159265f * (float)s / (float)(steps > 1 ? steps : 1)));
     const float c1 = 1.0f - std::pow(b1, (float)M->step), c2 = 1.0f - std::pow(b2, (float)M->step);
-    k_adam<<<(MLP_NPARAM + 255) / 256, 256>>>(MLP_NPARAM, M->w, M->m, M->v, M->g, M->wr, lr_s, b1, b2, c1, c2);
+    k_reduce_gradients<true><<<GT_PART / 32, 256>>>(gradient_grid(batch), M->part, M->g, batch, M->w, M->m, M->v, M->wr,
+                                                    lr_s, b1, b2, c1, c2);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) rc = cueva_fail(CUEVA_ERR_CUDA, cudaGetErrorString(e));
   }
   if (!rc && loss_out) {
-    cudaError_t e = cudaMemcpy(loss_out, M->loss, sizeof(float), cudaMemcpyDeviceToHost);
+    cudaError_t e = cudaMemcpy(loss_out, M->g + MLP_NPARAM, sizeof(float), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) rc = cueva_fail(CUEVA_ERR_CUDA, cudaGetErrorString(e));
   }
   if (X) cudaFree(X);
@@ -558,21 +698,15 @@ int32_t cueva_mlp_gradients(cueva_mlp* M, const double* d_cons, const double* d_
                             float* loss_out) {
   if (!M || n <= 0 || !d_cons || !d_p || !grads) return cueva_fail(CUEVA_ERR_ARG, "bad arguments");
   TRY(cudaSetDevice(M->dev));
-  if (int32_t e = ensure_batch(M, n)) return e;
-  float *X = nullptr, *T = nullptr;
-  int32_t rc = features_of(n, d_cons, d_p, &X, &T);
-  if (!rc) {
-    k_gather<<<(n + 255) / 256, 256>>>(n, n, 0ull, 0, X, T, M->norm, M->Xb, M->Tb);
-    rc = forward_backward(M, n);
-  }
-  if (!rc) {
-    cudaError_t e = cudaMemcpy(grads, M->g, MLP_NPARAM * sizeof(float), cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess && loss_out) e = cudaMemcpy(loss_out, M->loss, sizeof(float), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) rc = cueva_fail(CUEVA_ERR_CUDA, cudaGetErrorString(e));
-  }
-  if (X) cudaFree(X);
-  if (T) cudaFree(T);
-  return rc;
+  if (int32_t e = forward_backward(M, n, n, 0ull, nullptr, nullptr, d_cons, d_p)) return e;
+  k_reduce_gradients<false><<<GT_PART / 32, 256>>>(gradient_grid(n), M->part, M->g, n, nullptr, nullptr, nullptr,
+                                                   nullptr, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f);
+  TRY(cudaGetLastError());
+  float host[MLP_NPARAM + 1];
+  TRY(cudaMemcpy(host, M->g, sizeof host, cudaMemcpyDeviceToHost));
+  std::memcpy(grads, host, MLP_NPARAM * sizeof(float));
+  if (loss_out) *loss_out = host[MLP_NPARAM];
+  return CUEVA_OK;
 }
 
 int32_t cueva_mlp_predict(cueva_mlp* M, const double* d_cons, int64_t n, double* d_pseed, int32_t tensor_cores) {
