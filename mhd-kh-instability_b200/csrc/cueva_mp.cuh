@@ -30,9 +30,19 @@ __device__ __forceinline__ T DMM(T x, T y) {
   const T m = fmin2(fabs(x), fabs(y));
   return (signbit(x) == signbit(y)) ? copysign(m, x) : T(0) * m;
 }
+// DMM for the monotonicity tests, with a plain zero where the signs differ:
+// the test's product is the same for finite arguments, and where an
+// argument is infinite or NaN the value under test is not finite or equals
+// an infinite u, so the test fails either way
+template <typename T>
+__device__ __forceinline__ T DMM_test(T x, T y) {
+  const T m = fmin2(fabs(x), fabs(y));
+  return (signbit(x) == signbit(y)) ? copysign(m, x) : T(0);
+}
 template <typename T>
 __device__ __forceinline__ T DM4(T w, T xx, T y, T z) {
-  const T m = fmin2(fmin2(fmin2(fabs(w), fabs(xx)), fabs(y)), fabs(z));
+  // (w and x are NaN whenever y or z is, so the order of the minima is free)
+  const T m = fmin2(fmin2(fabs(w), fabs(xx)), fmin2(fabs(y), fabs(z)));
   const bool sw = signbit(w);
   const bool first = signbit(xx) == sw;
   if (first && signbit(y) == sw && signbit(z) == sw) return copysign(m, w);
@@ -53,19 +63,23 @@ __device__ __forceinline__ T mc_slope(T fa, T fb) {
   return (signbit(fa) == signbit(fb)) ? copysign(m, fa) : T(0) * m;
 }
 
-// unlimited left value at k+1/2 (SH97 eq. 2.1 / 2.31) around register index C
+// unlimited left value at k+1/2 (SH97 eq. 2.1 / 2.31) around register index C.
+// A product with 2 or 4 is exact, so it is taken in one FMA with the
+// neighbouring term: same rounding, one operation less (with DMM_test and
+// the halves of the HLLC fluxes: 2048 x 4096 step 15.43 -> 14.89 ms, B200).
 template <int RM, int C, typename T, int N>
 __device__ __forceinline__ T mp_vorp(const T (&u)[N]) {
   if constexpr (RM == 0) {
     const T b1 = T(1.0 / 60.0);
-    return b1 * (T(2.0) * u[C - 2] - T(13.0) * u[C - 1] + T(47.0) * u[C] + T(27.0) * u[C + 1] - T(3.0) * u[C + 2]);
+    return b1 * (fma_rn(T(2.0), u[C - 2], -(T(13.0) * u[C - 1])) + T(47.0) * u[C] + T(27.0) * u[C + 1] -
+                 T(3.0) * u[C + 2]);
   } else if constexpr (RM == 1) {
     const T b1 = T(1.0 / 420.0);
-    return b1 * (-T(3.0) * u[C - 3] + T(25.0) * u[C - 2] - T(101.0) * u[C - 1] + T(319.0) * u[C] +
-                 T(214.0) * u[C + 1] - T(38.0) * u[C + 2] + T(4.0) * u[C + 3]);
+    return b1 * fma_rn(T(4.0), u[C + 3], -T(3.0) * u[C - 3] + T(25.0) * u[C - 2] - T(101.0) * u[C - 1] +
+                                             T(319.0) * u[C] + T(214.0) * u[C + 1] - T(38.0) * u[C + 2]);
   } else {
     const T b1 = T(1.0 / 2520.0);
-    return b1 * (T(4.0) * u[C - 4] - T(41.0) * u[C - 3] + T(199.0) * u[C - 2] - T(641.0) * u[C - 1] +
+    return b1 * (fma_rn(T(4.0), u[C - 4], -(T(41.0) * u[C - 3])) + T(199.0) * u[C - 2] - T(641.0) * u[C - 1] +
                  T(1879.0) * u[C] + T(1375.0) * u[C + 1] - T(305.0) * u[C + 2] + T(55.0) * u[C + 3] -
                  T(5.0) * u[C + 4]);
   }
@@ -75,14 +89,15 @@ template <int RM, int C, typename T, int N>
 __device__ __forceinline__ T mp_vorm(const T (&u)[N]) {
   if constexpr (RM == 0) {
     const T b1 = T(1.0 / 60.0);
-    return b1 * (-T(3.0) * u[C - 2] + T(27.0) * u[C - 1] + T(47.0) * u[C] - T(13.0) * u[C + 1] + T(2.0) * u[C + 2]);
+    return b1 * fma_rn(T(2.0), u[C + 2],
+                       -T(3.0) * u[C - 2] + T(27.0) * u[C - 1] + T(47.0) * u[C] - T(13.0) * u[C + 1]);
   } else if constexpr (RM == 1) {
     const T b1 = T(1.0 / 420.0);
-    return b1 * (-T(3.0) * u[C + 3] + T(25.0) * u[C + 2] - T(101.0) * u[C + 1] + T(319.0) * u[C] +
-                 T(214.0) * u[C - 1] - T(38.0) * u[C - 2] + T(4.0) * u[C - 3]);
+    return b1 * fma_rn(T(4.0), u[C - 3], -T(3.0) * u[C + 3] + T(25.0) * u[C + 2] - T(101.0) * u[C + 1] +
+                                             T(319.0) * u[C] + T(214.0) * u[C - 1] - T(38.0) * u[C - 2]);
   } else {
     const T b1 = T(1.0 / 2520.0);
-    return b1 * (T(4.0) * u[C + 4] - T(41.0) * u[C + 3] + T(199.0) * u[C + 2] - T(641.0) * u[C + 1] +
+    return b1 * (fma_rn(T(4.0), u[C + 4], -(T(41.0) * u[C + 3])) + T(199.0) * u[C + 2] - T(641.0) * u[C + 1] +
                  T(1879.0) * u[C] + T(1375.0) * u[C - 1] - T(305.0) * u[C - 2] + T(55.0) * u[C - 3] -
                  T(5.0) * u[C - 4]);
   }
@@ -90,77 +105,55 @@ __device__ __forceinline__ T mp_vorm(const T (&u)[N]) {
 
 // up(k) for the cell at register index C (mp5.f95:104-136) in two steps:
 // mp_up_fast gives the unlimited value vorp and whether it passes the
-// monotonicity test (then vorp is up(k)); mp_up_lim gives the limited value
-// of a vorp that failed it.  mp_up chains them; the interface pairs below
-// take all their tests first (independent chains for the scheduler) and
-// limit only the values that failed.  The operations are the same.
+// monotonicity test (then vorp is up(k)).  The interface pairs below take all
+// their tests first (independent chains for the scheduler) and limit only
+// the values that failed, together.
 template <int RM, int C, typename T, int N>
 __device__ __forceinline__ T mp_up_fast(const T (&u)[N], bool& ok) {
   const T alpha = T(2.0), epsm = T(1.0e-10);
   const T du0 = u[C] - u[C - 1];
   const T du1 = u[C + 1] - u[C];
   const T vorp = mp_vorp<RM, C>(u);
-  const T vmpp = u[C] + DMM(du1, alpha * du0);
+  const T vmpp = u[C] + DMM_test(du1, alpha * du0);
   ok = (vorp - u[C]) * (vorp - vmpp) <= epsm;
   return vorp;
 }
-template <int RM, int C, typename T, int N>
-__device__ __forceinline__ T mp_up_lim(const T (&u)[N], T vorp) {
-  const T alpha = T(2.0), b2 = T(4.0 / 3.0);
-  const T du0 = u[C] - u[C - 1];
-  const T d2m = u[C - 2] - T(2.0) * u[C - 1] + u[C];
-  const T d20 = u[C - 1] - T(2.0) * u[C] + u[C + 1];
-  const T d2p = u[C] - T(2.0) * u[C + 1] + u[C + 2];
-  const T dm4jph = DM4(T(4.0) * d20 - d2p, T(4.0) * d2p - d20, d20, d2p);
-  const T dm4jmh = DM4(T(4.0) * d20 - d2m, T(4.0) * d2m - d20, d20, d2m);
-  const T vul = u[C] + alpha * du0;
-  const T vav = T(0.5) * (u[C] + u[C + 1]);
-  const T vmd = vav - T(0.5) * dm4jph;
-  const T vlc = u[C] + T(0.5) * du0 + b2 * dm4jmh;
-  const T vmin = fmax2(fmin2(fmin2(u[C], u[C + 1]), vmd), fmin2(fmin2(u[C], vul), vlc));
-  const T vmax = fmin2(fmax2(fmax2(u[C], u[C + 1]), vmd), fmax2(fmax2(u[C], vul), vlc));
-  return vorp + DMM(vmin - vorp, vmax - vorp);
-}
-template <int RM, int C, typename T, int N>
-__device__ __forceinline__ T mp_up(const T (&u)[N]) {
-  bool ok;
-  const T v = mp_up_fast<RM, C>(u, ok);
-  return ok ? v : mp_up_lim<RM, C>(u, v);
-}
-
-// um(k) for the cell at register index C (mp5.f95:142-167), same two steps
+// um(k) for the cell at register index C (mp5.f95:142-167), same first step
 template <int RM, int C, typename T, int N>
 __device__ __forceinline__ T mp_um_fast(const T (&u)[N], bool& ok) {
   const T alpha = T(2.0), epsm = T(1.0e-10);
   const T du0 = u[C] - u[C - 1];
   const T du1 = u[C + 1] - u[C];
   const T vorm = mp_vorm<RM, C>(u);
-  const T vmpm = u[C] + DMM(-du0, -alpha * du1);
+  const T vmpm = u[C] + DMM_test(-du0, -alpha * du1);
   ok = (vorm - u[C]) * (vorm - vmpm) <= epsm;
   return vorm;
 }
+// the limited values of an interface pair, both sides in one go: their
+// chains are independent (latency), and the curvature limiter in the middle
+// of the face is the same number for both (DM4 is symmetric in what its
+// arguments are permuted by)
 template <int RM, int C, typename T, int N>
-__device__ __forceinline__ T mp_um_lim(const T (&u)[N], T vorm) {
+__device__ __forceinline__ void mp_lim_pair(const T (&u)[N], T& L, T& R, bool okL, bool okR) {
   const T alpha = T(2.0), b2 = T(4.0 / 3.0);
-  const T du1 = u[C + 1] - u[C];
-  const T d2m = u[C - 2] - T(2.0) * u[C - 1] + u[C];
-  const T d20 = u[C - 1] - T(2.0) * u[C] + u[C + 1];
-  const T d2p = u[C] - T(2.0) * u[C + 1] + u[C + 2];
-  const T dm4jph = DM4(T(4.0) * d20 - d2p, T(4.0) * d2p - d20, d20, d2p);
-  const T dm4jmh = DM4(T(4.0) * d20 - d2m, T(4.0) * d2m - d20, d20, d2m);
-  const T vul = u[C] - alpha * du1;
-  const T vav = T(0.5) * (u[C] + u[C - 1]);
-  const T vmd = vav - T(0.5) * dm4jmh;
-  const T vlc = u[C] - T(0.5) * du1 + b2 * dm4jph;
-  const T vmin = fmax2(fmin2(fmin2(u[C], u[C - 1]), vmd), fmin2(fmin2(u[C], vul), vlc));
-  const T vmax = fmin2(fmax2(fmax2(u[C], u[C - 1]), vmd), fmax2(fmax2(u[C], vul), vlc));
-  return vorm + DMM(vmin - vorm, vmax - vorm);
-}
-template <int RM, int C, typename T, int N>
-__device__ __forceinline__ T mp_um(const T (&u)[N]) {
-  bool ok;
-  const T v = mp_um_fast<RM, C>(u, ok);
-  return ok ? v : mp_um_lim<RM, C>(u, v);
+  const T duL = u[C] - u[C - 1], duR = u[C + 2] - u[C + 1];
+  const T dA = u[C - 2] - T(2.0) * u[C - 1] + u[C];
+  const T dB = u[C - 1] - T(2.0) * u[C] + u[C + 1];
+  const T dC = u[C] - T(2.0) * u[C + 1] + u[C + 2];
+  const T dD = u[C + 1] - T(2.0) * u[C + 2] + u[C + 3];
+  const T dm4L = DM4(T(4.0) * dB - dA, T(4.0) * dA - dB, dB, dA);
+  const T dm4M = DM4(T(4.0) * dB - dC, T(4.0) * dC - dB, dB, dC);
+  const T dm4R = DM4(T(4.0) * dC - dD, T(4.0) * dD - dC, dC, dD);
+  const T av = T(0.5) * (u[C] + u[C + 1]), md = av - T(0.5) * dm4M;
+  const T lo = fmin2(u[C], u[C + 1]), hi = fmax2(u[C], u[C + 1]);   // u[C + 1], u[C] on the right: equal values
+  const T ulL = u[C] + alpha * duL, lcL = u[C] + T(0.5) * duL + b2 * dm4L;
+  const T ulR = u[C + 1] - alpha * duR, lcR = u[C + 1] - T(0.5) * duR + b2 * dm4R;
+  const T mnL = fmax2(fmin2(lo, md), fmin2(fmin2(u[C], ulL), lcL));
+  const T mxL = fmin2(fmax2(hi, md), fmax2(fmax2(u[C], ulL), lcL));
+  const T mnR = fmax2(fmin2(lo, md), fmin2(fmin2(u[C + 1], ulR), lcR));
+  const T mxR = fmin2(fmax2(hi, md), fmax2(fmax2(u[C + 1], ulR), lcR));
+  if (!okL) L = L + DMM(mnL - L, mxL - L);
+  if (!okR) R = R + DMM(mnR - R, mxR - R);
 }
 
 // interface pair: u holds cells i-R .. i+1+R; returns L = up(i), R = um(i+1)
@@ -172,11 +165,11 @@ __device__ __forceinline__ void mp_pair(const T (&u)[N], T& L, T& R) {
   bool okL, okR;
   L = mp_up_fast<RM, C>(u, okL);
   R = mp_um_fast<RM, C + 1>(u, okR);
-  if (!okL) L = mp_up_lim<RM, C>(u, L);
-  if (!okR) R = mp_um_lim<RM, C + 1>(u, R);
+  if (!(okL && okR)) mp_lim_pair<RM, C>(u, L, R, okL, okR);
 }
-// up(k), um(k) of the cells at C and C + 1 (the positivity-fixed pairs),
-// the four tests first
+// up(k), um(k) of the cells at C and C + 1 (the positivity-fixed pairs), the
+// four tests first, then the limited values of those that failed with the
+// three curvature limiters they share
 template <int RM, int C, typename T, int N>
 __device__ __forceinline__ void mp_quad(const T (&u)[N], T& up0, T& um0, T& up1, T& um1) {
   bool o0, o1, o2, o3;
@@ -184,10 +177,28 @@ __device__ __forceinline__ void mp_quad(const T (&u)[N], T& up0, T& um0, T& up1,
   um0 = mp_um_fast<RM, C>(u, o1);
   up1 = mp_up_fast<RM, C + 1>(u, o2);
   um1 = mp_um_fast<RM, C + 1>(u, o3);
-  if (!o0) up0 = mp_up_lim<RM, C>(u, up0);
-  if (!o1) um0 = mp_um_lim<RM, C>(u, um0);
-  if (!o2) up1 = mp_up_lim<RM, C + 1>(u, up1);
-  if (!o3) um1 = mp_um_lim<RM, C + 1>(u, um1);
+  if (o0 && o1 && o2 && o3) return;
+  const T alpha = T(2.0), b2 = T(4.0 / 3.0);
+  const T dA = u[C - 2] - T(2.0) * u[C - 1] + u[C];
+  const T dB = u[C - 1] - T(2.0) * u[C] + u[C + 1];
+  const T dC = u[C] - T(2.0) * u[C + 1] + u[C + 2];
+  const T dD = u[C + 1] - T(2.0) * u[C + 2] + u[C + 3];
+  const T dm4L = DM4(T(4.0) * dB - dA, T(4.0) * dA - dB, dB, dA);
+  const T dm4M = DM4(T(4.0) * dB - dC, T(4.0) * dC - dB, dB, dC);
+  const T dm4R = DM4(T(4.0) * dC - dD, T(4.0) * dD - dC, dC, dD);
+  // value w of the cell value c towards its neighbour n: slope d on the far
+  // side (signed towards n), curvatures near and far
+  auto limit = [&](T w, T c, T n, T d, T nearc, T farc) {
+    const T md = T(0.5) * (c + n) - T(0.5) * nearc;
+    const T ul = c + alpha * d, lc = c + T(0.5) * d + b2 * farc;
+    const T mn = fmax2(fmin2(fmin2(c, n), md), fmin2(fmin2(c, ul), lc));
+    const T mx = fmin2(fmax2(fmax2(c, n), md), fmax2(fmax2(c, ul), lc));
+    return w + DMM(mn - w, mx - w);
+  };
+  if (!o0) up0 = limit(up0, u[C], u[C + 1], u[C] - u[C - 1], dm4M, dm4L);
+  if (!o1) um0 = limit(um0, u[C], u[C - 1], -(u[C + 1] - u[C]), dm4L, dm4M);
+  if (!o2) up1 = limit(up1, u[C + 1], u[C + 2], u[C + 1] - u[C], dm4R, dm4M);
+  if (!o3) um1 = limit(um1, u[C + 1], u[C], -(u[C + 2] - u[C + 1]), dm4M, dm4R);
 }
 
 // pair for the p / rho slots: the positivity fix-up of mp5.f95:177-216 makes

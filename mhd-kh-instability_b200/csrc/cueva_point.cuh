@@ -161,25 +161,26 @@ __device__ __forceinline__ double e2b2_half(const C2PIn& in) {
 // Roots of 4c^3 - 3c = y, y in (-1, 1): by the triple-angle identity
 // cos 3a = 4 cos^3 a - 3 cos a they are cos((acos y + 2 pi k)/3); c0 in
 // (1/2, 1) and c1 in (-1, -1/2) by monotone Newton from c = 1 and c = -1,
-// c2 from -(c0 + c1) (the roots sum to zero) polished by Newton.
-__device__ __forceinline__ void chebyshev_roots(double y, double& c0, double& c1, double& c2) {
-  double c = 1.0;
+// c2 from -(c0 + c1) (the roots sum to zero) polished by Newton.  The caller
+// asks for a root at a time: the first is nearly always the one it takes.
+__device__ __forceinline__ double chebyshev_newton(double c, double y) {
+  return c - ((4.0 * c * c - 3.0) * c - y) / (12.0 * c * c - 3.0);
+}
+__device__ __forceinline__ double chebyshev_root(int r, double y, double c0, double c1) {
+  if (r == 2) {
+    double c = -(c0 + c1);
+#pragma unroll 1
+    for (int it = 0; it < 3; ++it) c = chebyshev_newton(c, y);
+    return c;
+  }
+  double c = r == 0 ? 1.0 : -1.0;
+#pragma unroll 1
   for (int it = 0; it < 80; ++it) {
-    const double cn = c - ((4.0 * c * c - 3.0) * c - y) / (12.0 * c * c - 3.0);
-    if (!(cn < c)) break;
+    const double cn = chebyshev_newton(c, y);
+    if (!(r == 0 ? cn < c : cn > c)) break;
     c = cn;
   }
-  c0 = c;
-  c = -1.0;
-  for (int it = 0; it < 80; ++it) {
-    const double cn = c - ((4.0 * c * c - 3.0) * c - y) / (12.0 * c * c - 3.0);
-    if (!(cn > c)) break;
-    c = cn;
-  }
-  c1 = c;
-  c = -(c0 + c1);
-  for (int it = 0; it < 3; ++it) c = c - ((4.0 * c * c - 3.0) * c - y) / (12.0 * c * c - 3.0);
-  c2 = c;
+  return c;
 }
 // x^(1/3), x >= 0: Newton cube root on the mantissa (frexp/ldexp are exact)
 // d_2 + 2 z_1 under the square root of the one-real-root branch of
@@ -201,7 +202,7 @@ __device__ __forceinline__ double cbrt_newton(double x) {
   const int q = (e - r) / 3;
   m = ldexp(m, r);
   double y = 1.0;
-#pragma unroll
+#pragma unroll 1
   for (int it = 0; it < 8; ++it) y = y - (y * y * y - m) / (3.0 * y * y);
   return ldexp(y, q);
 }
@@ -234,21 +235,24 @@ __device__ __forceinline__ uint32_t c2p_cardano(const C2PIn& in, double gamma, d
   const double R_1 = (2.0 * pw3(e) - 9.0 * e * f + 27.0 * g) / 54.0;
   double s = 0.0, t = 0.0, det = 0.0, z_1 = 0.0;
   if (pw2(R_1) < pw3(Q_1)) {
-    double ca, cb, cc;   // cos(T/3), cos((T+2pi)/3), cos((T-2pi)/3), T = acos(R/|Q|^1.5)
-    chebyshev_roots(R_1 / fabs(sqrt(pw3(Q_1))), ca, cb, cc);
+    // cos(T/3), cos((T+2pi)/3), cos((T-2pi)/3), T = acos(R/|Q|^1.5), in turn
+    const double y = R_1 / fabs(sqrt(pw3(Q_1)));
     const double sq = fabs(sqrt(Q_1));
-    const double zs[3] = {-2.0 * sq * ca - e / 3.0, -2.0 * sq * cb - e / 3.0, -2.0 * sq * cc - e / 3.0};
+    double c0 = 0.0, c1 = 0.0;
     bool found = false;
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-      if (found) break;
-      const double s_1 = d_2 + 2.0 * zs[r];
-      const double t_1 = pw2(zs[r]) + 2.0 * d_2 * zs[r] + pw2(d_2) - d_0;
+#pragma unroll 1
+    for (int r = 0; r < 3 && !found; ++r) {
+      const double c = chebyshev_root(r, y, c0, c1);
+      if (r == 0) c0 = c;
+      else c1 = c;
+      const double z = -2.0 * sq * c - e / 3.0;
+      const double s_1 = d_2 + 2.0 * z;
+      const double t_1 = pw2(z) + 2.0 * d_2 * z + pw2(d_2) - d_0;
       if (s_1 >= 0.0 && t_1 >= 0.0) {
         s = fabs(sqrt(s_1));
         t = fabs(sqrt(t_1));
-        det = pw2(s) - 4.0 * (d_2 + zs[r] - t);
-        z_1 = zs[r];
+        det = pw2(s) - 4.0 * (d_2 + z - t);
+        z_1 = z;
         if (det < 0.0) st |= ST_C2P_FAIL;
         found = true;
       }

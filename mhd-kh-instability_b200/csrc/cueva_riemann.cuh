@@ -104,8 +104,9 @@ __device__ __forceinline__ Phys<T> physical(const Side<T>& s, T gamma, T W) {
   const T Bn = X::Bn(s), Bt1 = X::Bt1(s), Bt2 = X::Bt2(s);
   f.FD = s.D * vn;
   f.Ftau = (Bt2 * Et1 - Bt1 * Et2) + hW2 * vn;
-  if constexpr (PS) f.FSn = -pw2(En) - pw2(Bn) + hW2 * pw2(vn) + T(0.5) * E2B2 + s.dp;
-  else f.FSn = -pw2(En) - pw2(Bn) + hW2 * pw2(vn) + T(0.5) * E2B2 + s.p;
+  const T FSn = fma_rn(T(0.5), E2B2, -pw2(En) - pw2(Bn) + hW2 * pw2(vn));   // half of E2B2 is exact
+  if constexpr (PS) f.FSn = FSn + s.dp;
+  else f.FSn = FSn + s.p;
   f.FSt1 = -En * Et1 - Bn * Bt1 + hW2 * vn * vt1;
   if constexpr (D == 0) f.FSt2 = -En * Et2 - Bn * Bt2 + hW2 * vn * vt2;
   else                  f.FSt2 = -En * Et2 - Bn * Bt2 + hW2 * vt2 * vn;   // FSyx: vx before vy
@@ -347,13 +348,14 @@ __device__ __forceinline__ void hllc_fluxes(const Side<T>& L, const Side<T>& R, 
   // tau, S receive the star correction; E, B, q keep the HLL fluxes.
   if (V > T(0.0) || V < T(0.0)) {
     const T k = V > T(0.0) ? omV : opV;
-    A[R_PSI] = psi_f + (k * (psiR - psiL)) * h;
-    A[R_PHI] = phi_f + (k * (phiR - phiL)) * h;
-    A[R_D] = D_f + k * (DR - DL) * h;
-    A[R_TAU] = tau_f + k * (tauR - tauL) * h;
-    A[R_SN] = Sn_f + k * (SnR - SnL) * h;
-    A[R_ST1] = St1_f + k * (St1R - St1L) * h;
-    A[R_ST2] = St2_f + k * (St2R - St2L) * h;
+    auto star = [&](T f, T r, T l) { return fma_rn(k * (r - l), h, f); };   // f + (k (r - l)) / 2
+    A[R_PSI] = star(psi_f, psiR, psiL);
+    A[R_PHI] = star(phi_f, phiR, phiL);
+    A[R_D] = star(D_f, DR, DL);
+    A[R_TAU] = star(tau_f, tauR, tauL);
+    A[R_SN] = star(Sn_f, SnR, SnL);
+    A[R_ST1] = star(St1_f, St1R, St1L);
+    A[R_ST2] = star(St2_f, St2R, St2L);
   } else if (V == T(0.0)) {
     A[R_D] = D_f; A[R_TAU] = tau_f; A[R_SN] = Sn_f; A[R_ST1] = St1_f; A[R_ST2] = St2_f;
   } else {
@@ -551,13 +553,14 @@ __device__ __forceinline__ void hllcmc_fluxes(const Side<T>& L, const Side<T>& R
   // v* == 0 the HLL fluxes; E, B and q keep the HLL fluxes throughout
   if (V > T(0.0) || V < T(0.0)) {
     const T k = V > T(0.0) ? omV : opV;
-    A[R_PSI] = psi_f + (k * (psiR - psiL)) * h;
-    A[R_PHI] = phi_f + (k * (phiR - phiL)) * h;
-    A[R_D] = D_f + k * (DR - DL) * h;
-    A[R_TAU] = tau_f + k * (tauR - tauL) * h;
-    A[R_SN] = Sn_f + k * (SnR - SnL) * h;
-    A[R_ST1] = St1_f + k * (St1R - St1L) * h;
-    A[R_ST2] = St2_f + k * (St2R - St2L) * h;
+    auto star = [&](T f, T r, T l) { return fma_rn(k * (r - l), h, f); };   // f + (k (r - l)) / 2
+    A[R_PSI] = star(psi_f, psiR, psiL);
+    A[R_PHI] = star(phi_f, phiR, phiL);
+    A[R_D] = star(D_f, DR, DL);
+    A[R_TAU] = star(tau_f, tauR, tauL);
+    A[R_SN] = star(Sn_f, SnR, SnL);
+    A[R_ST1] = star(St1_f, St1R, St1L);
+    A[R_ST2] = star(St2_f, St2R, St2L);
   } else if (!(V == T(0.0))) {
     st |= ST_HLLC_VSTAR;
 #pragma unroll
