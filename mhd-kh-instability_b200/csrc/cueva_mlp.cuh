@@ -111,14 +111,6 @@ __device__ __forceinline__ float mlp_forward(const MLPDevice& M, const float f[M
   return y;
 }
 
-// pressure seed of the network for a conserved state
-__device__ __forceinline__ double mlp_pressure_seed(const MLPDevice& M, const C2PIn& in) {
-  float f[MLP_IN];
-  c2p_features(in.D, in.tau, in.Sx, in.Sy, in.Sz, in.Ex, in.Ey, in.Ez, in.Bx, in.By, in.Bz, f);
-  const float y = mlp_forward(M, f) * M.sd_y + M.mu_y;
-  return in.D * (double)__expf(y);
-}
-
 // ---- warp-cooperative inference on the tensor cores ------------------------
 // A converged warp evaluates the network for its 32 states with
 // mma.sync.m16n8k16 (bf16 in, FP32 accumulate): two 16-row tiles, 8

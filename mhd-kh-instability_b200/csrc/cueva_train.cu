@@ -409,29 +409,163 @@ __global__ void k_round(int n, const float* w, float* wr) {
   if (i < n) wr[i] = __bfloat162float(__float2bfloat16(w[i]));
 }
 
-// batch con2prim: method 1 Cardano, 2 network seed + Newton (Cardano when it
-// fails), 3 Newton from seed[i]; iters[i] = Newton iterations (-1 failed,
-// 0 for Cardano)
-__global__ void k_c2p_batch(long long n, int method, double gamma, double eps1, const MLPDevice* M,
-                            const double* cons, const double* prev, const double* seed, double* out, int* iters) {
+// one state of the batch con2prim arrays
+__device__ __forceinline__ C2PIn batch_state(long long n, long long i, const double* __restrict__ cons,
+                                             const double* __restrict__ prev) {
+  return C2PIn{cons[i], cons[n + i], cons[2 * n + i], cons[3 * n + i], cons[4 * n + i], cons[5 * n + i],
+               cons[6 * n + i], cons[7 * n + i], cons[8 * n + i], cons[9 * n + i], cons[10 * n + i],
+               prev[2 * n + i], prev[3 * n + i], prev[4 * n + i], prev[i], prev[n + i]};
+}
+// Newton from p0, Cardano where it fails; iters[i] = Newton iterations (-1 failed)
+__device__ __forceinline__ void batch_recover(long long n, long long i, const C2PIn& in, double p0, double gamma,
+                                              double eps1, double* out, int* iters) {
+  C2POut o{};
+  const int it = c2p_newton(in, gamma, p0, o);
+  if (it < 0) c2p_cardano_ool(in, gamma, eps1, o, nullptr);
+  out[i] = o.rho; out[n + i] = o.p; out[2 * n + i] = o.vx; out[3 * n + i] = o.vy; out[4 * n + i] = o.vz;
+  if (iters) iters[i] = it;
+}
+
+// batch con2prim without the network: method 1 Cardano (iters 0), 3 Newton
+// from seed[i]
+__global__ void k_c2p_batch(long long n, int method, double gamma, double eps1, const double* __restrict__ cons,
+                            const double* __restrict__ prev, const double* __restrict__ seed, double* out, int* iters) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    C2PIn in{cons[i], cons[n + i], cons[2 * n + i], cons[3 * n + i], cons[4 * n + i], cons[5 * n + i],
-             cons[6 * n + i], cons[7 * n + i], cons[8 * n + i], cons[9 * n + i], cons[10 * n + i],
-             prev[2 * n + i], prev[3 * n + i], prev[4 * n + i], prev[i], prev[n + i]};
-    C2POut o{};
-    int it = 0;
+    const C2PIn in = batch_state(n, i, cons, prev);
     if (method == 1) {
+      C2POut o{};
       c2p_cardano(in, gamma, eps1, o, nullptr);
+      out[i] = o.rho; out[n + i] = o.p; out[2 * n + i] = o.vx; out[3 * n + i] = o.vy; out[4 * n + i] = o.vz;
+      if (iters) iters[i] = 0;
     } else {
-      // 2: the network's seed; 4: the network's or the previous pressure,
-      // whichever leaves the smaller residual; 3: the given seeds
-      const double p0 = (method == 2) ? mlp_pressure_seed(*M, in)
-                        : (method == 4) ? c2p_best_seed(in, gamma, mlp_pressure_seed(*M, in)) : seed[i];
-      it = c2p_newton(in, gamma, p0, o);
-      if (it < 0) c2p_cardano(in, gamma, eps1, o, nullptr);
+      batch_recover(n, i, in, seed[i], gamma, eps1, out, iters);
     }
-    out[i] = o.rho; out[n + i] = o.p; out[2 * n + i] = o.vx; out[3 * n + i] = o.vy; out[4 * n + i] = o.vz;
-    if (iters) iters[i] = it;
+  }
+}
+
+// batch con2prim with the FP32 network: method 2 its seed, 4 its seed or the
+// previous pressure, whichever leaves the smaller residual (Newton; Cardano
+// where it fails).
+//
+// A CTA takes tiles of 128 states.  Thread t prepares the features and
+// recovers state t; in between the two 64 x 64 layers run as register-tiled
+// FP32 matrix products (8 states x 8 outputs per thread, K = 64) from shared
+// memory, in place.  Every output is the sum of mlp_forward in the same
+// order (bias first, ascending k, one FMA each), so the seeds are the same
+// bits.  What bounds it: 8.6 k FMAs per state, 0.23 ms per million states at
+// the FP32 rate.  With one thread per state (mlp_forward) each weight was
+// loaded and widened again for every FMA: 1895 us for 10^6 states on a B200;
+// tiled 622 us; with two states per FMA instruction 600 us (the issue slots
+// go to the recovery's FP64 chains at 12 warps per SM).  mma.sync or tcgen05
+// would round the activations to bf16.
+constexpr int CN_ROWS = 128;
+struct C2PNet {
+  alignas(16) float w2t[MLP_H * MLP_H], w3t[MLP_H * MLP_H];   // [input][output]
+  alignas(16) float act[MLP_H * CN_ROWS];                     // [unit][state]
+  float w1[MLP_H * MLP_IN], w4[MLP_H], b1[MLP_H], b2[MLP_H], b3[MLP_H], b4;
+  float mu[MLP_IN], sd[MLP_IN], mu_y, sd_y;
+};
+
+// two FP32 FMAs in one instruction (each rounded as fmaf)
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+  unsigned long long d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+
+// act <- silu(W act + b): outputs 4 og + {0..3} and 32 + those, states 4 sg +
+// {0..3} and 64 + those, in pairs of states
+__device__ __forceinline__ void c2p_layer(float* act, const float* wt, const float* b) {
+  const int sg = threadIdx.x & 15, og = threadIdx.x >> 4;
+  unsigned long long z[8][4];
+#pragma unroll
+  for (int o = 0; o < 8; ++o) {
+    const float bo = b[(o >> 2) * 32 + 4 * og + (o & 3)];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) z[o][s] = pack2(bo, bo);
+  }
+#pragma unroll 4
+  for (int k = 0; k < MLP_H; ++k) {
+    const ulonglong2 a0 = *reinterpret_cast<const ulonglong2*>(act + k * CN_ROWS + 4 * sg);
+    const ulonglong2 a1 = *reinterpret_cast<const ulonglong2*>(act + k * CN_ROWS + 64 + 4 * sg);
+    const float4 w0 = *reinterpret_cast<const float4*>(wt + k * MLP_H + 4 * og);
+    const float4 w1 = *reinterpret_cast<const float4*>(wt + k * MLP_H + 32 + 4 * og);
+    const unsigned long long av[4] = {a0.x, a0.y, a1.x, a1.y};
+    const float wv[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+    for (int o = 0; o < 8; ++o) {
+      const unsigned long long w = pack2(wv[o], wv[o]);
+#pragma unroll
+      for (int s = 0; s < 4; ++s) z[o][s] = fma2(w, av[s], z[o][s]);
+    }
+  }
+  __syncthreads();   // every input has been read
+#pragma unroll
+  for (int o = 0; o < 8; ++o) {
+    float* row = act + ((o >> 2) * 32 + 4 * og + (o & 3)) * CN_ROWS + 4 * sg;
+    const float2 p0 = unpack2(z[o][0]), p1 = unpack2(z[o][1]), p2 = unpack2(z[o][2]), p3 = unpack2(z[o][3]);
+    *reinterpret_cast<float4*>(row) = make_float4(silu(p0.x), silu(p0.y), silu(p1.x), silu(p1.y));
+    *reinterpret_cast<float4*>(row + 64) = make_float4(silu(p2.x), silu(p2.y), silu(p3.x), silu(p3.y));
+  }
+  __syncthreads();
+}
+
+__global__ void __launch_bounds__(CN_ROWS, 3)
+k_c2p_network(long long n, int method, double gamma, double eps1, const MLPDevice* __restrict__ M,
+              const double* __restrict__ cons, const double* __restrict__ prev, double* out, int* iters) {
+  extern __shared__ __align__(16) unsigned char cn_smem[];
+  C2PNet& S = *reinterpret_cast<C2PNet*>(cn_smem);
+  const int t = threadIdx.x;
+  for (int e = t; e < MLP_H * MLP_H; e += CN_ROWS) {
+    const int o = e / MLP_H, k = e % MLP_H;
+    S.w2t[k * MLP_H + o] = __bfloat162float(M->W2[e]);
+    S.w3t[k * MLP_H + o] = __bfloat162float(M->W3[e]);
+  }
+  for (int e = t; e < MLP_H * MLP_IN; e += CN_ROWS) S.w1[e] = __bfloat162float(M->W1[e]);
+  if (t < MLP_H) {
+    S.w4[t] = __bfloat162float(M->W4[t]);
+    S.b1[t] = M->b1[t]; S.b2[t] = M->b2[t]; S.b3[t] = M->b3[t];
+    if (t < MLP_IN) { S.mu[t] = M->mu[t]; S.sd[t] = M->sd[t]; }
+    if (t == 0) { S.b4 = M->b4; S.mu_y = M->mu_y; S.sd_y = M->sd_y; }
+  }
+  __syncthreads();
+  const long long ntiles = (n + CN_ROWS - 1) / CN_ROWS;
+  for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const long long i0 = tile * CN_ROWS + t;
+    const long long i = i0 < n ? i0 : n - 1;   // threads past the end repeat the last state
+    const C2PIn in = batch_state(n, i, cons, prev);
+    float x[MLP_IN];
+    c2p_features(in.D, in.tau, in.Sx, in.Sy, in.Sz, in.Ex, in.Ey, in.Ez, in.Bx, in.By, in.Bz, x);
+#pragma unroll
+    for (int k = 0; k < MLP_IN; ++k) x[k] = (x[k] - S.mu[k]) / S.sd[k];
+#pragma unroll 4
+    for (int o = 0; o < MLP_H; ++o) {
+      float z = S.b1[o];
+#pragma unroll
+      for (int k = 0; k < MLP_IN; ++k) z = fmaf(S.w1[o * MLP_IN + k], x[k], z);
+      S.act[o * CN_ROWS + t] = silu(z);
+    }
+    __syncthreads();
+    c2p_layer(S.act, S.w2t, S.b2);
+    c2p_layer(S.act, S.w3t, S.b3);
+    float y = S.b4;
+#pragma unroll 8
+    for (int k = 0; k < MLP_H; ++k) y = fmaf(S.w4[k], S.act[k * CN_ROWS + t], y);
+    y = y * S.sd_y + S.mu_y;
+    const double p_net = in.D * (double)__expf(y);
+    const double p0 = method == 2 ? p_net : c2p_best_seed(in, gamma, p_net);
+    if (i0 < n) batch_recover(n, i, in, p0, gamma, eps1, out, iters);
+    __syncthreads();   // the activations have been read
   }
 }
 
@@ -744,8 +878,15 @@ int32_t cueva_c2p_batch(int32_t device, int32_t method, const cueva_mlp* M, doub
     return cueva_fail(CUEVA_ERR_ARG, "methods 2 and 4 need a trained network");
   if (method == 3 && !d_seed) return cueva_fail(CUEVA_ERR_ARG, "method 3 needs seeds");
   TRY(cudaSetDevice(device));
-  k_c2p_batch<<<grid_for(n), 256>>>(n, method, gamma, eps1, (method == 2 || method == 4) ? M->d_dev : nullptr, d_cons, d_prev, d_seed,
-                                    d_out, d_iters);
+  if (method == 2 || method == 4) {
+    // three CTAs per SM (66 KB of shared memory, up to 168 registers per thread)
+    TRY(cudaFuncSetAttribute(k_c2p_network, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(C2PNet)));
+    const long long tiles = (n + CN_ROWS - 1) / CN_ROWS;
+    k_c2p_network<<<(unsigned)std::min<long long>(tiles, 3 * 148), CN_ROWS, sizeof(C2PNet)>>>(
+        n, method, gamma, eps1, M->d_dev, d_cons, d_prev, d_out, d_iters);
+  } else {
+    k_c2p_batch<<<grid_for(n), 256>>>(n, method, gamma, eps1, d_cons, d_prev, d_seed, d_out, d_iters);
+  }
   TRY(cudaGetLastError());
   TRY(cudaDeviceSynchronize());
   return CUEVA_OK;
