@@ -70,7 +70,8 @@ template <> struct Dir<1> {
 };
 
 // physical fluxes of one reconstructed side, 16_hll_flow_mpx.f95:1464-1733;
-// h is the enthalpy density rho (1 + eps) + p
+// h is the enthalpy density rho (1 + eps) + p.  physical() leaves out FD =
+// D vn, the only one that needs a conserved fluid value.
 template <typename T> struct Phys { T FD, Ftau, FSn, FSt1, FSt2, h; };
 
 // Lorentz factor of the HLL / HLLC routines, 1 / sqrt(1 - (vx^2 + vy^2 + vz^2))
@@ -102,7 +103,6 @@ __device__ __forceinline__ Phys<T> physical(const Side<T>& s, T gamma, T W) {
   const T vn = X::vn(s), vt1 = X::vt1(s), vt2 = X::vt2(s);
   const T En = X::En(s), Et1 = X::Et1(s), Et2 = X::Et2(s);
   const T Bn = X::Bn(s), Bt1 = X::Bt1(s), Bt2 = X::Bt2(s);
-  f.FD = s.D * vn;
   f.Ftau = (Bt2 * Et1 - Bt1 * Et2) + hW2 * vn;
   const T FSn = fma_rn(T(0.5), E2B2, -pw2(En) - pw2(Bn) + hW2 * pw2(vn));   // half of E2B2 is exact
   if constexpr (PS) f.FSn = FSn + s.dp;
@@ -118,12 +118,20 @@ __device__ __forceinline__ Phys<T> physical(const Side<T>& s, T gamma) {
   return physical<D, PS>(s, gamma, lorentz(s));
 }
 
+// with FD, for a side whose conserved values are known
+template <int D, typename T>
+__device__ __forceinline__ Phys<T> physical_all(const Side<T>& s, T gamma, T W) {
+  Phys<T> f = physical<D>(s, gamma, W);
+  f.FD = s.D * Dir<D>::vn(s);
+  return f;
+}
+
 // fixed-speed (s1 = -1, s2 = +1) HLL combination
 // (s2*FL - s1*FR + s1*s2*(UR-UL))/(s2-s1) == 0.5*((FL+FR) - (UR-UL)) exactly
 template <typename T>
 __device__ __forceinline__ T hll(T FL, T FR, T UL, T UR) { return T(0.5) * ((FL + FR) - (UR - UL)); }
 
-// EM and charge fluxes (identical for HLL, HLLC and the HLLE EM part)
+// EM fluxes (identical for HLL, HLLC and the HLLE EM part)
 template <int D, typename T>
 __device__ __forceinline__ void em_fluxes(const Side<T>& L, const Side<T>& R, T* A) {
   using X = Dir<D>;
@@ -135,21 +143,34 @@ __device__ __forceinline__ void em_fluxes(const Side<T>& L, const Side<T>& R, T*
   A[R_EN] = hll(L.psi, R.psi, X::En(L), X::En(R));
   A[R_ET1] = hll(X::Bt2(L), X::Bt2(R), X::Et1(L), X::Et1(R));
   A[R_ET2] = T(0.5) * ((X::Bt1(L) + X::Bt1(R)) + (X::Et2(R) - X::Et2(L)));
-  A[R_Q] = hll(L.J, R.J, L.q, R.q);
 }
 
+// The MP flux routines below take the conserved fluid values (D, tau, S) from
+// `cons`: cons(role, l, r) reconstructs them when they are wanted, after the
+// physical fluxes, so that each pair is folded into its HLL state and flux at
+// once.  With every field reconstructed first, 40 FP64 face values were alive
+// around the last calls of the limiter (128 registers; k_stage HLLC spilled
+// 428 bytes, now 380).  Steps on a B200: 2048 x 4096 HLLC 14.41 -> 14.36 ms,
+// 700 x 1500 MP9 2.26 -> 2.22 ms, 1024 x 2048 mixed MP7 3.76 -> 3.72 ms.
+
 // PS: split pressure (see physical); A[R_SN] then lacks the reference
-// pressure, which the caller adds in FP64
-template <int D, bool PS = false, typename T>
-__device__ __forceinline__ void hll_fluxes(const Side<T>& L, const Side<T>& R, T gamma, T* A) {
+// pressure, which the caller adds in FP64.  The charge flux is the caller's.
+template <int D, bool PS = false, typename T, class CONS>
+__device__ __forceinline__ void hll_fluxes(const Side<T>& L, const Side<T>& R, T gamma, T* A, const CONS& cons) {
   using X = Dir<D>;
   em_fluxes<D>(L, R, A);
   const Phys<T> fl = physical<D, PS>(L, gamma), fr = physical<D, PS>(R, gamma);
-  A[R_D] = hll(fl.FD, fr.FD, L.D, R.D);
-  A[R_TAU] = hll(fl.Ftau, fr.Ftau, L.tau, R.tau);
-  A[R_SN] = hll(fl.FSn, fr.FSn, X::Sn(L), X::Sn(R));
-  A[R_ST1] = hll(fl.FSt1, fr.FSt1, X::St1(L), X::St1(R));
-  A[R_ST2] = hll(fl.FSt2, fr.FSt2, X::St2(L), X::St2(R));
+  T l, r;
+  cons(R_D, l, r);
+  A[R_D] = hll(l * X::vn(L), r * X::vn(R), l, r);
+  cons(R_TAU, l, r);
+  A[R_TAU] = hll(fl.Ftau, fr.Ftau, l, r);
+  cons(R_SN, l, r);
+  A[R_SN] = hll(fl.FSn, fr.FSn, l, r);
+  cons(R_ST1, l, r);
+  A[R_ST1] = hll(fl.FSt1, fr.FSt1, l, r);
+  cons(R_ST2, l, r);
+  A[R_ST2] = hll(fl.FSt2, fr.FSt2, l, r);
 }
 
 // HLL of the second-order MCL routine, 16_hll_flow_mcl.f95:1014-1396 (Sp = 1):
@@ -177,7 +198,7 @@ __device__ __forceinline__ void mcl_fluxes(const Side<T>& L, const Side<T>& R, c
     return sigma * W * (X::En(s) + vrotB - Edotv * X::vn(s)) + s.q * X::vn(s);
   };
   A[R_Q] = hll(jn(L, WL), jn(R, WR), L.q, R.q);
-  const Phys<T> fl = physical<D>(L, gamma, WL), fr = physical<D>(R, gamma, WR);
+  const Phys<T> fl = physical_all<D>(L, gamma, WL), fr = physical_all<D>(R, gamma, WR);
   A[R_D] = hll(fl.FD, fr.FD, L.D, R.D);
   A[R_TAU] = hll(fl.Ftau, fr.Ftau, L.tau, R.tau);
   A[R_SN] = hll(fl.FSn, fr.FSn, X::Sn(L), X::Sn(R));
@@ -270,9 +291,9 @@ __device__ __forceinline__ T hllc_vel(T a, T b, T c, T rt, uint32_t& st) {
 // momentum fluxes and the star pressure lack pc0, which cancels in every
 // star-state difference; the contact-speed quadratic takes the full flux.
 // A[R_SN] then lacks pc0, which the caller adds in FP64.
-template <int D, bool PS = false, typename T>
+template <int D, bool PS = false, typename T, class CONS>
 __device__ __forceinline__ void hllc_fluxes(const Side<T>& L, const Side<T>& R, T gamma, T* A, uint32_t& st,
-                                            T* vstar = nullptr, T pc0 = T(0)) {
+                                            const CONS& cons, T* vstar = nullptr, T pc0 = T(0)) {
   using X = Dir<D>;
   em_fluxes<D>(L, R, A);
   const Phys<T> fl = physical<D, PS>(L, gamma), fr = physical<D, PS>(R, gamma);
@@ -286,21 +307,25 @@ __device__ __forceinline__ void hllc_fluxes(const Side<T>& L, const Side<T>& R, 
   const T Bn_hll = h * (((X::Bn(R) + X::Bn(L)) + L.phi) - R.phi);
   const T Bt1_hll = h * (((X::Bt1(R) + X::Bt1(L)) - X::Et2(L)) + X::Et2(R));
   const T Bt2_hll = h * (((X::Bt2(R) + X::Bt2(L)) + X::Et1(L)) - X::Et1(R));
-  const T D_hll = h * (((R.D + L.D) + fl.FD) - fr.FD);
-  const T tau_hll = h * (((R.tau + L.tau) + fl.Ftau) - fr.Ftau);
-  const T Sn_hll = h * (((X::Sn(R) + X::Sn(L)) + fl.FSn) - fr.FSn);
-  const T St1_hll = h * (((X::St1(R) + X::St1(L)) + fl.FSt1) - fr.FSt1);
-  const T St2_hll = h * (((X::St2(R) + X::St2(L)) + fl.FSt2) - fr.FSt2);
   // HLL fluxes that enter the star states (:2904-3100)
   const T psi_f = A[R_PSI];
   const T phi_f = A[R_PHI];
   const T En_f = A[R_EN];
   const T Bn_f = A[R_BN];
-  const T D_f = hll(fl.FD, fr.FD, L.D, R.D);
-  const T tau_f = hll(fl.Ftau, fr.Ftau, L.tau, R.tau);
-  const T Sn_f = hll(fl.FSn, fr.FSn, X::Sn(L), X::Sn(R));
-  const T St1_f = hll(fl.FSt1, fr.FSt1, X::St1(L), X::St1(R));
-  const T St2_f = hll(fl.FSt2, fr.FSt2, X::St2(L), X::St2(R));
+  // fluid values, states and fluxes
+  auto fold = [&](int role, T Fl, T Fr, T& U, T& F) {
+    T l, r;
+    cons(role, l, r);
+    if (role == R_D) { Fl = l * Fl; Fr = r * Fr; }   // FD = D vn
+    U = h * (((r + l) + Fl) - Fr);
+    F = hll(Fl, Fr, l, r);
+  };
+  T D_hll, D_f, tau_hll, tau_f, Sn_hll, Sn_f, St1_hll, St1_f, St2_hll, St2_f;
+  fold(R_D, X::vn(L), X::vn(R), D_hll, D_f);
+  fold(R_TAU, fl.Ftau, fr.Ftau, tau_hll, tau_f);
+  fold(R_SN, fl.FSn, fr.FSn, Sn_hll, Sn_f);
+  fold(R_ST1, fl.FSt1, fr.FSt1, St1_hll, St1_f);
+  fold(R_ST2, fl.FSt2, fr.FSt2, St2_hll, St2_f);
   // star E, B = HLL averages; cross product E x B by role (:3144-3160)
   const T ErotB_n = Bt2_hll * Et1_hll - Bt1_hll * Et2_hll;
   const T ErotB_t1 = Bn_hll * Et2_hll - Bt2_hll * En_hll;
@@ -387,12 +412,12 @@ __device__ __forceinline__ void hlle_bounds(const Side<T>& s, T h, T gamma, T& l
 }
 
 // PS: split pressure with reference pressure pc0, as in hllc_fluxes
-template <int D, bool PS = false, typename T>
+template <int D, bool PS = false, typename T, class CONS>
 __device__ __forceinline__ void hlle_fluxes(const Side<T>& L, const Side<T>& R, T gamma, T* A, uint32_t& st,
-                                            T pc0 = T(0)) {
+                                            const CONS& cons, T pc0 = T(0)) {
   using X = Dir<D>;
   em_fluxes<D>(L, R, A);   // psi, phi, E, B; the charge flux is replaced below
-  const Phys<T> fl = physical<D, PS>(L, gamma, lorentz_hlle(L)), fr = physical<D, PS>(R, gamma, lorentz_hlle(R));
+  Phys<T> fl = physical<D, PS>(L, gamma, lorentz_hlle(L)), fr = physical<D, PS>(R, gamma, lorentz_hlle(R));
   const T h = T(0.5);
   // fixed-speed HLL states of E and B (the star E, B)
   const T En_hll = h * (((X::En(R) + X::En(L)) + L.psi) - R.psi);
@@ -411,18 +436,21 @@ __device__ __forceinline__ void hlle_fluxes(const Side<T>& L, const Side<T>& R, 
   if (fabs(s1) > T(1.0)) s1 = fmax2(T(-1.0) + eps2, fmin2(T(1.0) - eps2, s1));
   if (fabs(s2) > T(1.0)) s2 = fmax2(T(-1.0) + eps2, fmin2(T(1.0) - eps2, s2));
   // fluid HLL states and HLLE fluxes with the bounds
-  const T D_hll = (s2 * R.D - s1 * L.D + fl.FD - fr.FD) / (s2 - s1);
-  const T tau_hll = (s2 * R.tau - s1 * L.tau + fl.Ftau - fr.Ftau) / (s2 - s1);
-  const T Sn_hll = (s2 * X::Sn(R) - s1 * X::Sn(L) + fl.FSn - fr.FSn) / (s2 - s1);
-  const T St1_hll = (s2 * X::St1(R) - s1 * X::St1(L) + fl.FSt1 - fr.FSt1) / (s2 - s1);
-  const T St2_hll = (s2 * X::St2(R) - s1 * X::St2(L) + fl.FSt2 - fr.FSt2) / (s2 - s1);
   auto hlle = [&](T FL, T FR, T UL, T UR) { return (s2 * FL - s1 * FR + s1 * s2 * (UR - UL)) / (s2 - s1); };
   const T q_f = hlle(L.J, R.J, L.q, R.q);
-  const T D_f = hlle(fl.FD, fr.FD, L.D, R.D);
-  const T tau_f = hlle(fl.Ftau, fr.Ftau, L.tau, R.tau);
-  const T Sn_f = hlle(fl.FSn, fr.FSn, X::Sn(L), X::Sn(R));
-  const T St1_f = hlle(fl.FSt1, fr.FSt1, X::St1(L), X::St1(R));
-  const T St2_f = hlle(fl.FSt2, fr.FSt2, X::St2(L), X::St2(R));
+  auto fold = [&](int role, T Fl, T Fr, T& U, T& F) {
+    T l, r;
+    cons(role, l, r);
+    if (role == R_D) { fl.FD = Fl = l * Fl; fr.FD = Fr = r * Fr; }   // FD = D vn
+    U = (s2 * r - s1 * l + Fl - Fr) / (s2 - s1);
+    F = hlle(Fl, Fr, l, r);
+  };
+  T D_hll, D_f, tau_hll, tau_f, Sn_hll, Sn_f, St1_hll, St1_f, St2_hll, St2_f;
+  fold(R_D, X::vn(L), X::vn(R), D_hll, D_f);
+  fold(R_TAU, fl.Ftau, fr.Ftau, tau_hll, tau_f);
+  fold(R_SN, fl.FSn, fr.FSn, Sn_hll, Sn_f);
+  fold(R_ST1, fl.FSt1, fr.FSt1, St1_hll, St1_f);
+  fold(R_ST2, fl.FSt2, fr.FSt2, St2_hll, St2_f);
   // contact speed of the HLLC quadratic, with the HLLE states and fluxes
   const T ErotB_n = Bt2_hll * Et1_hll - Bt1_hll * Et2_hll;
   const T ErotB_t1 = Bn_hll * Et2_hll - Bt2_hll * En_hll;
@@ -496,7 +524,7 @@ __device__ __forceinline__ void hllcmc_fluxes(const Side<T>& L, const Side<T>& R
                                               T* vstar = nullptr) {
   using X = Dir<D>;
   mcl_fluxes<D>(L, R, m_et2, m_bt1, gamma, sigma, A);   // fixed-speed HLL fluxes of every role
-  const Phys<T> fl = physical<D>(L, gamma, lorentz_hlle(L)), fr = physical<D>(R, gamma, lorentz_hlle(R));
+  const Phys<T> fl = physical_all<D>(L, gamma, lorentz_hlle(L)), fr = physical_all<D>(R, gamma, lorentz_hlle(R));
   const T h = T(0.5);
   const T psi_hll = h * (((R.psi + L.psi) + X::En(L)) - X::En(R));
   const T phi_hll = h * (((R.phi + L.phi) + X::Bn(L)) - X::Bn(R));
@@ -598,7 +626,7 @@ __device__ __forceinline__ void hllemc_fluxes(const Side<T>& L, const Side<T>& R
   const T Bt1_hll = h * (((X::Bt1(R) + X::Bt1(L)) + m_et2[0]) - m_et2[1]);
   const T Bt2_hll = h * (((X::Bt2(R) + X::Bt2(L)) + X::Et1(L)) - X::Et1(R));
   const T WL = lorentz_hlle(L), WR = lorentz_hlle(R);
-  const Phys<T> fl = physical<D>(L, gamma, WL), fr = physical<D>(R, gamma, WR);
+  const Phys<T> fl = physical_all<D>(L, gamma, WL), fr = physical_all<D>(R, gamma, WR);
   auto jn = [&](const Side<T>& s, T W) {
     const T vrotB = X::Bt2(s) * X::vt1(s) - X::Bt1(s) * X::vt2(s);
     const T Edotv = s.Ex * s.vx + s.Ey * s.vy + s.Ez * s.vz;

@@ -552,6 +552,11 @@ __device__ __forceinline__ uint32_t face_flux(const ACC& acc, const FacePre<T>* 
       }
     }
   }
+  // charge and current first: the fixed-speed routines need only their flux
+  rec(5 + Q_Q, L.q, Rs.q);
+  rec(19, L.J, Rs.J);
+  T q_flux = T(0);
+  if constexpr (SOLVER != 6) q_flux = hll(L.J, Rs.J, L.q, Rs.q);
   if constexpr (kEmF64<T, SOLVER>) {
     // mixed precision: psi, phi, E and B are reconstructed as differences
     // from the cell's FP64 value (the MP limiters are translation-equivariant:
@@ -593,21 +598,22 @@ __device__ __forceinline__ uint32_t face_flux(const ACC& acc, const FacePre<T>* 
     rec(5 + Q_BY, L.By, Rs.By);
     rec(5 + Q_BZ, L.Bz, Rs.Bz);
   }
-  rec(5 + Q_Q, L.q, Rs.q);
-  rec(5 + Q_D, L.D, Rs.D);
-  rec(5 + Q_TAU, L.tau, Rs.tau);
-  rec(5 + Q_SX, L.Sx, Rs.Sx);
-  rec(5 + Q_SY, L.Sy, Rs.Sy);
-  rec(5 + Q_SZ, L.Sz, Rs.Sz);
-  rec(19, L.J, Rs.J);
+  // D, tau, S when the flux routine wants them (see hll_fluxes)
+  auto cons = [&](int role, T& l, T& r) {
+    const int f = role == R_D ? 5 + Q_D
+                  : role == R_TAU ? 5 + Q_TAU
+                                  : 5 + Q_SX + (D == 0 ? role - R_SN : (role - R_SN + 1) % 3);   // n, t1, t2
+    rec(f, l, r);
+  };
   const T gamma = T(gamma_d);
   T vstar = T(0);
   constexpr bool PS = kSplitP<T, SOLVER>;
   auto riemann = [&](T* A) {
-    if constexpr (SOLVER == 5) hll_fluxes<D, PS>(L, Rs, gamma, A);
-    else if constexpr (SOLVER == 6) hlle_fluxes<D, PS>(L, Rs, gamma, A, stt, T(pc0));
+    if constexpr (SOLVER != 6) A[R_Q] = q_flux;
+    if constexpr (SOLVER == 5) hll_fluxes<D, PS>(L, Rs, gamma, A, cons);
+    else if constexpr (SOLVER == 6) hlle_fluxes<D, PS>(L, Rs, gamma, A, stt, cons, T(pc0));
     else if constexpr (SOLVER == 7)
-      hllc_fluxes<D, PS>(L, Rs, gamma, A, stt, kEmF64<T, SOLVER> ? &vstar : nullptr, T(pc0));
+      hllc_fluxes<D, PS>(L, Rs, gamma, A, stt, cons, kEmF64<T, SOLVER> ? &vstar : nullptr, T(pc0));
   };
   if constexpr (kEmF64<T, SOLVER>) {
     T A[NROLE];
