@@ -240,6 +240,7 @@ struct cueva_ctx {
   int nkslot = 0;
   int kslot_of[8];        // slot of K_m (0-based m) or -1
   StageShape shape;       // tile height, CTAs and tiles of the two stage launches
+  int wide_rows = 0;      // the grid's stage tiles are those of the wide form with this many warps
   int cur = 0, qin = 0;
   bool primed = false;
   double* bound[CUEVA_NFIELDS] = {};
@@ -466,7 +467,9 @@ int32_t cueva_ctx_create(const cueva_params* p, cueva_ctx** out) {
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->dev);
   I.block_count[LK_XUPD] = xupd_tiles(c->imax, c->jmax, FACE_ROWS);
   I.block_count[LK_YFACE] = yface_tiles(c->imax, c->jmax, FACE_ROWS);
-  I.seg_rows = stage_seg_rows(c->imax, c->jmax, FACE_ROWS, 2 * nsm);
+  const int grid[2] = {c->imax, c->jmax};
+  c->wide_rows = c->shape.wide_rows = stage_wide_rows(p->flux_solver, grid, 1, nsm);
+  I.seg_rows = c->wide_rows ? c->wide_rows - 1 : stage_seg_rows(c->imax, c->jmax, FACE_ROWS, 2 * nsm);
   I.block_count[LK_STAGE] = stage_tiles(c->imax, c->jmax, I.seg_rows);
   c->shape.rows = FACE_ROWS;
   for (int k : {LK_XUPD, LK_YFACE, LK_STAGE}) {
@@ -526,6 +529,8 @@ int32_t cueva_set_stage_kernel(cueva_ctx* c, int32_t fused) {
   CUDA_TRY(cudaStreamSynchronize(c->stream));
   destroy_graphs(c);
   c->shape.fused = fused != 0;
+  // the two-kernel form on request; MP7 and MP9 have no fused form to choose and keep theirs
+  if (stage_fused_available(c->P.rec_mp, c->P.flux_solver)) c->shape.wide_rows = fused ? c->wide_rows : 0;
   return CUEVA_OK;
 }
 
@@ -732,7 +737,7 @@ int32_t cueva_profile_steps(cueva_ctx* c, int32_t nsteps, double ms_out[3], int3
       if (ce == cudaSuccess) ce = cudaEventSynchronize(ev[2]);
       if (ce != cudaSuccess) { rc = fail(CUEVA_ERR_CUDA, cudaGetErrorString(ce)); break; }
       for (int k = 0; k < 2; ++k) {
-        if (k == 0 && c->shape.fused) continue;   // no separate y-face launch
+        if (k == 0 && (c->shape.fused || c->shape.wide_rows)) continue;   // no separate y-face launch
         float ms = 0.f;
         cudaEventElapsedTime(&ms, ev[k], ev[k + 1]);
         ms_out[k] += ms;
@@ -1436,12 +1441,17 @@ void ens_destroy_graphs(cueva_ens* e) {
 // tile ranges for a tile height and the launch grid for a CTA count per SM
 int32_t ens_apply_shape(cueva_ens* e, int rows, int ctas_per_sm) {
   int begin[4] = {0, 0, 0, 0};
+  std::vector<int> grids;
+  for (const InstDesc& I : e->I) { grids.push_back(I.imax); grids.push_back(I.jmax); }
+  const int wide = rows == FACE_ROWS && ctas_per_sm == 0
+                       ? stage_wide_rows(e->P0.flux_solver, grids.data(), e->n, e->num_sms) : 0;
+  e->shape.wide_rows = wide;
   for (int k = 0; k < e->n; ++k) {
     InstDesc& I = e->I[k];
     I.block_count[LK_XUPD] = xupd_tiles(I.imax, I.jmax, rows);
     I.block_count[LK_YFACE] = yface_tiles(I.imax, I.jmax, rows);
     I.block_count[LK_C2P] = c2p_tiles(I.imax, I.jmax);
-    I.seg_rows = stage_seg_rows(I.imax, I.jmax, FACE_ROWS, 2 * e->num_sms);
+    I.seg_rows = wide ? wide - 1 : stage_seg_rows(I.imax, I.jmax, FACE_ROWS, 2 * e->num_sms);
     I.block_count[LK_STAGE] = stage_tiles(I.imax, I.jmax, I.seg_rows);
     for (int t = 0; t < 4; ++t) { I.block_begin[t] = begin[t]; begin[t] += I.block_count[t]; }
   }

@@ -207,6 +207,7 @@ __device__ __forceinline__ int map_idx(int i, int n, int periodic) {
 // update 31 points per row; ROWS is 8 or 4), 256 threads for the pointwise
 // kernels
 constexpr int FACE_ROWS = 8;   // default tile height
+constexpr int WIDE_ROWS = 12;  // most warps of a tile of the fused stage kernel's wide form
 constexpr int NFACE = 14;   // interface fluxes per face (the Riemann roles)
 constexpr int POINT_THREADS = 256;
 enum LaunchKind { LK_XUPD = 0, LK_YFACE = 1, LK_C2P = 2, LK_STAGE = 3 };
@@ -220,6 +221,9 @@ struct StageShape {
   int grid[4] = {0, 0, 0, 0};
   int ntiles[4] = {0, 0, 0, 0};
   bool fused = false;
+  // not 0: one k_stage per stage in its wide form, with this many warps per tile
+  // (ntiles[LK_STAGE] tiles of one row less): see stage_wide_rows
+  int wide_rows = 0;
 };
 
 // tiles of one instance for a tile height (x tiles: 31 points by rows)

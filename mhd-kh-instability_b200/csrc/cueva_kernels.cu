@@ -198,6 +198,24 @@ bool stage_fused_available(int rec_mp, int solver) {
   }
 }
 
+int stage_wide_rows(int solver, const int* grids, int ngrids, int num_sms) {
+  // The fewest warps per tile (from one per scheduler on) whose tiles find an
+  // SM each: the stage of a small grid is one tile's time, and that falls with
+  // the warps that share an SM's FP64 pipes.
+  // Stage times on a B200 without / with it: 64 x 32 MP5 HLL 45 / 39 us (always 8
+  // warps a tile: 49), MP7 HLLC 60 (two kernels) / 39; 200 x 100 MP5 44 / 38;
+  // 256 x 128 MP5 HLL 42.9 / 40.7, MP9 HLLC 55 / 43.  Where no height up to 12
+  // finds an SM for every tile, two CTAs of 8 warps per SM are as good: 320 x
+  // 160 MP5 HLL 45.9 / 45.8 us.
+  if (solver < 5) return 0;
+  for (int rows = 4; rows <= WIDE_ROWS; ++rows) {
+    long long tiles = 0;
+    for (int k = 0; k < ngrids; ++k) tiles += stage_tiles(grids[2 * k], grids[2 * k + 1], rows - 1);
+    if (tiles <= num_sms) return rows;
+  }
+  return 0;
+}
+
 int stage_seg_rows(int imax, int jmax, int rows, int slots) {
   // A tile of nb bands updates nb * rows - 1 grid rows (its first band also
   // computes the faces below the segment) and costs about nb band times; the

@@ -39,6 +39,9 @@ cudaError_t launch_stage(int rec_mp, int solver, int prec, const StageShape& sh,
 // whether the fused stage kernel k_stage exists for this reconstruction and
 // flux routine (tile height FACE_ROWS)
 bool stage_fused_available(int rec_mp, int solver);
+// warps per tile of the fused kernel's wide form for a launch over these grids
+// (pairs of imax, jmax), or 0 where it does not apply
+int stage_wide_rows(int solver, const int* grids, int ngrids, int num_sms);
 // grid rows per fused-stage tile for a grid: a multiple of rows, so that the
 // launch has enough tiles to balance over `slots` resident CTAs
 int stage_seg_rows(int imax, int jmax, int rows, int slots);

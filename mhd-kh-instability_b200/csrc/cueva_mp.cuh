@@ -238,13 +238,53 @@ __device__ __forceinline__ void mp_pair_pos_delta(const T (&u)[N], double c0, T&
   R = um1;
 }
 
+// two fields' pairs side by side: twice the independent chains of mp_pair,
+// for kernels whose warps have nothing else to wait on
+template <int RM, typename T, int N>
+__device__ __forceinline__ void mp_pair2(const T (&u)[N], const T (&v)[N], T& uL, T& uR, T& vL, T& vR) {
+  constexpr int C = MPR<RM>::R;
+  bool a, b, c, d;
+  uL = mp_up_fast<RM, C>(u, a);
+  uR = mp_um_fast<RM, C + 1>(u, b);
+  vL = mp_up_fast<RM, C>(v, c);
+  vR = mp_um_fast<RM, C + 1>(v, d);
+  if (!(a && b && c && d)) {
+    mp_lim_pair<RM, C>(u, uL, uR, a, b);
+    mp_lim_pair<RM, C>(v, vL, vR, c, d);
+  }
+}
+
 // Out-of-line entry points.  A sweep thread reconstructs ~45 slots per grid
 // point; inlining the limiter 45 times made the kernel larger than the
 // instruction cache (ncu: "no instruction" was the top stall).  One copy of
 // each limiter body is called with the stencil values in registers.
 template <typename T> struct Pair { T L, R; };
 
+template <typename T> struct Pair2 { T uL, uR, vL, vR; };
+
 template <int RM, typename T> struct MPCall;
+// two fields in one call (MP5 and MP7; the arguments of two MP9 stencils no
+// longer fit the registers of a call)
+template <int RM, typename T> struct MPCall2;
+template <typename T> struct MPCall2<0, T> {
+  static __device__ __noinline__ Pair2<T> pair(T a0, T a1, T a2, T a3, T a4, T a5, T b0, T b1, T b2, T b3, T b4, T b5) {
+    const T u[6] = {a0, a1, a2, a3, a4, a5}, v[6] = {b0, b1, b2, b3, b4, b5};
+    Pair2<T> p; mp_pair2<0>(u, v, p.uL, p.uR, p.vL, p.vR); return p;
+  }
+  static __device__ __forceinline__ Pair2<T> call(const T (&u)[6], const T (&v)[6]) {
+    return pair(u[0], u[1], u[2], u[3], u[4], u[5], v[0], v[1], v[2], v[3], v[4], v[5]);
+  }
+};
+template <typename T> struct MPCall2<1, T> {
+  static __device__ __noinline__ Pair2<T> pair(T a0, T a1, T a2, T a3, T a4, T a5, T a6, T a7, T b0, T b1, T b2, T b3,
+                                               T b4, T b5, T b6, T b7) {
+    const T u[8] = {a0, a1, a2, a3, a4, a5, a6, a7}, v[8] = {b0, b1, b2, b3, b4, b5, b6, b7};
+    Pair2<T> p; mp_pair2<1>(u, v, p.uL, p.uR, p.vL, p.vR); return p;
+  }
+  static __device__ __forceinline__ Pair2<T> call(const T (&u)[8], const T (&v)[8]) {
+    return pair(u[0], u[1], u[2], u[3], u[4], u[5], u[6], u[7], v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7]);
+  }
+};
 template <typename T> struct MPCall<0, T> {
   static __device__ __noinline__ Pair<T> pair(T a0, T a1, T a2, T a3, T a4, T a5) {
     const T u[6] = {a0, a1, a2, a3, a4, a5};

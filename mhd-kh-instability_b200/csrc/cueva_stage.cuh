@@ -299,7 +299,8 @@ constexpr bool kSplitP = kEmF64<T, SV> && mixed_split_p(SV);
 // flux of one face from its stencil accessor (16_hll_flow_mpx.f95 /
 // 16_hllc_flow_mpx.f95 for one interface); returns status bits.  With PRE
 // the primitive slots come from *pre instead of being reconstructed here.
-template <int RM, int SOLVER, typename T, int D, bool PRE, class ACC>
+// WIDE: two fields at a time where a two-field call exists (k_stage's wide form).
+template <int RM, int SOLVER, typename T, int D, bool PRE, bool WIDE = false, class ACC>
 __device__ __forceinline__ uint32_t face_flux(const ACC& acc, const FacePre<T>* pre, double gamma_d, double sigma_d,
                                               flux_t<T, SOLVER> (&F)[NROLE]) {
   constexpr int R = MPR<RM>::R, NS = 2 * R + 2;
@@ -312,6 +313,19 @@ __device__ __forceinline__ uint32_t face_flux(const ACC& acc, const FacePre<T>* 
     for (int q = 0; q < NS; ++q) u[q] = nrm(f, q);
     const Pair<T> p = MPCall<RM, T>::template call<false>(u);
     L = p.L; Rv = p.R;
+  };
+  constexpr bool kTwo = WIDE && RM <= 1;
+  auto rec2 = [&](int fa, T& La, T& Ra, int fb, T& Lb, T& Rb) {
+    if constexpr (kTwo) {
+      T u[NS], v[NS];
+#pragma unroll
+      for (int q = 0; q < NS; ++q) { u[q] = nrm(fa, q); v[q] = nrm(fb, q); }
+      const Pair2<T> p = MPCall2<RM, T>::call(u, v);
+      La = p.uL; Ra = p.uR; Lb = p.vL; Rb = p.vR;
+    } else {
+      rec(fa, La, Ra);
+      rec(fb, Lb, Rb);
+    }
   };
   auto recp = [&](int f, T& L, T& Rv) {
     T u[NS];
@@ -499,8 +513,7 @@ __device__ __forceinline__ uint32_t face_flux(const ACC& acc, const FacePre<T>* 
     L.rho = pre->rhoL; Rs.rho = pre->rhoR;
     if constexpr (kSplitP<T, SOLVER>) { L.dp = pre->dpL; Rs.dp = pre->dpR; pc0 = pre->pc0; }
   } else {
-    rec(0, L.vx, Rs.vx);
-    rec(1, L.vy, Rs.vy);
+    rec2(0, L.vx, Rs.vx, 1, L.vy, Rs.vy);
     rec(2, L.vz, Rs.vz);
     if constexpr (kSplitP<T, SOLVER>) {
       pc0 = nrmd(3, R);
@@ -553,8 +566,7 @@ __device__ __forceinline__ uint32_t face_flux(const ACC& acc, const FacePre<T>* 
     }
   }
   // charge and current first: the fixed-speed routines need only their flux
-  rec(5 + Q_Q, L.q, Rs.q);
-  rec(19, L.J, Rs.J);
+  rec2(5 + Q_Q, L.q, Rs.q, 19, L.J, Rs.J);
   T q_flux = T(0);
   if constexpr (SOLVER != 6) q_flux = hll(L.J, Rs.J, L.q, Rs.q);
   if constexpr (kEmF64<T, SOLVER>) {
@@ -572,14 +584,24 @@ __device__ __forceinline__ uint32_t face_flux(const ACC& acc, const FacePre<T>* 
       const Pair<T> p = MPCall<RM, T>::template call<false>(u);
       Lv = c0 + double(p.L); Rv = c0 + double(p.R);
     };
-    rec_delta(5 + Q_PSI, Ld.psi, Rd.psi);
-    rec_delta(5 + Q_PHI, Ld.phi, Rd.phi);
-    rec_delta(5 + Q_EX, Ld.Ex, Rd.Ex);
-    rec_delta(5 + Q_EY, Ld.Ey, Rd.Ey);
-    rec_delta(5 + Q_EZ, Ld.Ez, Rd.Ez);
-    rec_delta(5 + Q_BX, Ld.Bx, Rd.Bx);
-    rec_delta(5 + Q_BY, Ld.By, Rd.By);
-    rec_delta(5 + Q_BZ, Ld.Bz, Rd.Bz);
+    auto rec_delta2 = [&](int fa, double& La, double& Ra, int fb, double& Lb, double& Rb) {
+      if constexpr (kTwo) {
+        const double ca = nrmd(fa, R), cb = nrmd(fb, R);
+        T u[NS], v[NS];
+#pragma unroll
+        for (int q = 0; q < NS; ++q) { u[q] = T(nrmd(fa, q) - ca); v[q] = T(nrmd(fb, q) - cb); }
+        const Pair2<T> p = MPCall2<RM, T>::call(u, v);
+        La = ca + double(p.uL); Ra = ca + double(p.uR);
+        Lb = cb + double(p.vL); Rb = cb + double(p.vR);
+      } else {
+        rec_delta(fa, La, Ra);
+        rec_delta(fb, Lb, Rb);
+      }
+    };
+    rec_delta2(5 + Q_PSI, Ld.psi, Rd.psi, 5 + Q_PHI, Ld.phi, Rd.phi);
+    rec_delta2(5 + Q_EX, Ld.Ex, Rd.Ex, 5 + Q_EY, Ld.Ey, Rd.Ey);
+    rec_delta2(5 + Q_EZ, Ld.Ez, Rd.Ez, 5 + Q_BX, Ld.Bx, Rd.Bx);
+    rec_delta2(5 + Q_BY, Ld.By, Rd.By, 5 + Q_BZ, Ld.Bz, Rd.Bz);
     double Ad[NROLE];
     em_fluxes<D>(Ld, Rd, Ad);
 #pragma unroll
@@ -589,21 +611,22 @@ __device__ __forceinline__ uint32_t face_flux(const ACC& acc, const FacePre<T>* 
     Rs.psi = T(Rd.psi); Rs.phi = T(Rd.phi); Rs.Ex = T(Rd.Ex); Rs.Ey = T(Rd.Ey); Rs.Ez = T(Rd.Ez);
     Rs.Bx = T(Rd.Bx); Rs.By = T(Rd.By); Rs.Bz = T(Rd.Bz);
   } else {
-    rec(5 + Q_PSI, L.psi, Rs.psi);
-    rec(5 + Q_PHI, L.phi, Rs.phi);
-    rec(5 + Q_EX, L.Ex, Rs.Ex);
-    rec(5 + Q_EY, L.Ey, Rs.Ey);
-    rec(5 + Q_EZ, L.Ez, Rs.Ez);
-    rec(5 + Q_BX, L.Bx, Rs.Bx);
-    rec(5 + Q_BY, L.By, Rs.By);
-    rec(5 + Q_BZ, L.Bz, Rs.Bz);
+    rec2(5 + Q_PSI, L.psi, Rs.psi, 5 + Q_PHI, L.phi, Rs.phi);
+    rec2(5 + Q_EX, L.Ex, Rs.Ex, 5 + Q_EY, L.Ey, Rs.Ey);
+    rec2(5 + Q_EZ, L.Ez, Rs.Ez, 5 + Q_BX, L.Bx, Rs.Bx);
+    rec2(5 + Q_BY, L.By, Rs.By, 5 + Q_BZ, L.Bz, Rs.Bz);
   }
   // D, tau, S when the flux routine wants them (see hll_fluxes)
+  auto cons_field = [](int role) {
+    return role == R_D ? 5 + Q_D
+           : role == R_TAU ? 5 + Q_TAU
+                           : 5 + Q_SX + (D == 0 ? role - R_SN : (role - R_SN + 1) % 3);   // n, t1, t2
+  };
+  T nextL = T(0), nextR = T(0);   // the second field of a two-field call, asked for next
   auto cons = [&](int role, T& l, T& r) {
-    const int f = role == R_D ? 5 + Q_D
-                  : role == R_TAU ? 5 + Q_TAU
-                                  : 5 + Q_SX + (D == 0 ? role - R_SN : (role - R_SN + 1) % 3);   // n, t1, t2
-    rec(f, l, r);
+    if (kTwo && (role == R_TAU || role == R_ST1)) { l = nextL; r = nextR; }
+    else if (kTwo && role != R_ST2) rec2(cons_field(role), l, r, cons_field(role + 1), nextL, nextR);
+    else rec(cons_field(role), l, r);
   };
   const T gamma = T(gamma_d);
   T vstar = T(0);
@@ -999,6 +1022,10 @@ struct RingGeom {
   static constexpr int RING = NR * ROWSZ;
   static constexpr int YF = (ROWS + 1) * NROLE * 32;   // y-flux face rows x roles x lanes
   static constexpr size_t bytes() { return sizeof(double) * (size_t)(RING + YF); }
+  // of a one-band tile of `rows` warps (k_stage's wide form)
+  static constexpr size_t bytes(int rows) {
+    return sizeof(double) * ((size_t)(rows + 2 * R + 1) * ROWSZ + (size_t)(rows + 1) * NROLE * 32);
+  }
   // ring row of grid row r (r > -16 NR)
   static __device__ __forceinline__ int slot(int r) { return (int)((unsigned)(r + 16 * NR) % (unsigned)NR); }
 };
@@ -1006,6 +1033,9 @@ struct RingGeom {
 // 228 KB of shared memory (MP5 and the MC slopes)
 template <int RM>
 constexpr bool kFused = RingGeom<RM, FACE_ROWS>::bytes() <= 113 * 1024;
+// the wide form of the MP flux routines: one CTA of up to WIDE_ROWS warps per SM
+template <int RM, int SV>
+constexpr bool kWide = SV >= 5 && RingGeom<RM, WIDE_ROWS>::bytes(WIDE_ROWS) <= 224 * 1024;
 
 // first staged column of a strip (see RingGeom::LONG)
 template <int R>
@@ -1041,15 +1071,17 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
                : "memory");
 }
 
-// copies grid rows ra .. rb of the strip into their ring rows: with bulk,
+// copies grid rows ra .. rb of the strip into their ring rows (of a one-band
+// tile: rows counted from row0): with bulk,
 // one bulk copy per field and row, spread over all the CTA's threads
 // (completion on bar, which the caller waits for), else element by element
 // through the ghost maps
 // (columns i0-R .. ilast+R+1; the caller waits with cp.async.wait_all)
 template <int RM, int ROWS>
 __device__ __forceinline__ void ring_fill(const InstDesc& I, const StageArgs& sa, double* ring, int i0, int ilast,
-                                          int ra, int rb, int tid, bool bulk, uint64_t* bar) {
+                                          int ra, int rb, int tid, int nthr, int row0, bool bulk, uint64_t* bar) {
   using G = RingGeom<RM, ROWS>;
+  auto slot = [&](int r) { return ROWS == WIDE_ROWS ? r - row0 : G::slot(r); };
   constexpr int R = G::R, LONG = G::LONG;
   const long long fs = I.fstride;
   const double* __restrict__ prim = I.prim[sa.cur];
@@ -1061,25 +1093,25 @@ __device__ __forceinline__ void ring_fill(const InstDesc& I, const StageArgs& sa
     const int n = (rb - ra + 1) * NF_RING;
     constexpr uint32_t kRowBytes = LONG * sizeof(double);
     uint32_t mine = 0;
-    for (int e = tid; e < n; e += 32 * ROWS) mine += kRowBytes;
+    for (int e = tid; e < n; e += nthr) mine += kRowBytes;
     // the ring rows being replaced were read through the generic proxy
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     mbar_arrive_expect_tx(bar, mine);
-    for (int e = tid; e < n; e += 32 * ROWS) {
+    for (int e = tid; e < n; e += nthr) {
       const int r = e / NF_RING, f = e - r * NF_RING, row = ra + r;
       const double* src = ring_field(prim, Q, fs, f) + (long long)map_idx(row, I.jmax, I.bc_y) * I.pitch + cs;
-      bulk_g2s(ring + G::slot(row) * G::ROWSZ + f * LONG, src, kRowBytes, bar);
+      bulk_g2s(ring + slot(row) * G::ROWSZ + f * LONG, src, kRowBytes, bar);
     }
     return;
   }
   const int cfirst = i0 - R - cs, clast = ilast + R + 1 - cs;   // needed ring columns
   const int n = (rb - ra + 1) * LONG;
-  for (int e = tid; e < n; e += 32 * ROWS) {
+  for (int e = tid; e < n; e += nthr) {
     const int r = e / LONG, c = e - r * LONG;
     if (c < cfirst || c > clast) continue;
     const int row = ra + r;
     const long long off = (long long)map_idx(row, I.jmax, I.bc_y) * I.pitch + map_idx(cs + c, I.imax, I.bc_x);
-    double* dst = ring + G::slot(row) * G::ROWSZ + c;
+    double* dst = ring + slot(row) * G::ROWSZ + c;
     cp_async8(dst + 0 * LONG, prim + P_VX * fs + off);
     cp_async8(dst + 1 * LONG, prim + P_VY * fs + off);
     cp_async8(dst + 2 * LONG, prim + P_VZ * fs + off);
@@ -1138,16 +1170,25 @@ __device__ __forceinline__ void pressure_pair(const ACC& a, FacePre<T>& pre) {
 // fall-back of 16_hll_flow_mpx.f95:1393-1462: if any of the four
 // reconstructions is superluminal, both faces take cell (i, j) on the left
 // and cell (i-1, j) (x) or (i, j-1) (y) on the right
-template <int RM, typename T, class AX, class AY>
+template <int RM, typename T, bool WIDE, class AX, class AY>
 __device__ __forceinline__ void point_velocities(const AX& ax, const AY& ay, T (&xL)[3], T (&xR)[3], T (&yL)[3],
                                                  T (&yR)[3]) {
   constexpr int R = MPR<RM>::R;
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    const Pair<T> px = rec_acc<RM, T, false>(ax, c);
-    xL[c] = px.L; xR[c] = px.R;
-    const Pair<T> py = rec_acc<RM, T, false>(ay, c);
-    yL[c] = py.L; yR[c] = py.R;
+    if constexpr (WIDE && RM <= 1) {
+      constexpr int NS = 2 * R + 2;
+      T u[NS], v[NS];
+#pragma unroll
+      for (int q = 0; q < NS; ++q) { u[q] = T(ax.n(c, q)); v[q] = T(ay.n(c, q)); }
+      const Pair2<T> p = MPCall2<RM, T>::call(u, v);
+      xL[c] = p.uL; xR[c] = p.uR; yL[c] = p.vL; yR[c] = p.vR;
+    } else {
+      const Pair<T> px = rec_acc<RM, T, false>(ax, c);
+      xL[c] = px.L; xR[c] = px.R;
+      const Pair<T> py = rec_acc<RM, T, false>(ay, c);
+      yL[c] = py.L; yR[c] = py.R;
+    }
   }
   const T V2xl = pw2(xL[0]) + pw2(xL[1]) + pw2(xL[2]);
   const T V2xr = pw2(xR[0]) + pw2(xR[1]) + pw2(xR[2]);
@@ -1167,7 +1208,7 @@ __device__ __forceinline__ void point_velocities(const AX& ax, const AY& ay, T (
 // that the caller reloads before it stores the y fluxes there) and yneg tells
 // whether a raw y density face value is negative (the x density fix-up of
 // 16_hllc_flow_mpx.f95:2663-2690 looks at the y pair first)
-template <int RM, int SOLVER, typename T, int ROWS>
+template <int RM, int SOLVER, typename T, int ROWS, bool WIDE>
 __device__ __forceinline__ uint32_t fused_yface(const RingAcc<RM, ROWS, 0>& ax, const RingAcc<RM, ROWS, 1>& ay,
                                                 const InstDesc& I, volatile double* xstash, bool& yneg,
                                                 flux_t<T, SOLVER> (&F)[NROLE]) {
@@ -1177,7 +1218,7 @@ __device__ __forceinline__ uint32_t fused_yface(const RingAcc<RM, ROWS, 0>& ax, 
     FacePre<T> py;
     {
       T xL[3], xR[3];
-      point_velocities<RM, T>(ax, ay, xL, xR, py.vL, py.vR);
+      point_velocities<RM, T, WIDE>(ax, ay, xL, xR, py.vL, py.vR);
       if (xstash) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) { xstash[c * 32] = double(xL[c]); xstash[(3 + c) * 32] = double(xR[c]); }
@@ -1194,14 +1235,14 @@ __device__ __forceinline__ uint32_t fused_yface(const RingAcc<RM, ROWS, 0>& ax, 
         else py.rhoR = r10;
       }
     }
-    return face_flux<RM, SOLVER, T, 1, true>(ay, &py, I.gamma, I.sigma, F);
+    return face_flux<RM, SOLVER, T, 1, true, WIDE>(ay, &py, I.gamma, I.sigma, F);
   } else {
-    return face_flux<RM, SOLVER, T, 1, false>(ay, (const FacePre<T>*)nullptr, I.gamma, I.sigma, F);
+    return face_flux<RM, SOLVER, T, 1, false, WIDE>(ay, (const FacePre<T>*)nullptr, I.gamma, I.sigma, F);
   }
 }
 
 // x face (i+1/2, j) of point (i, j); xv = the velocity slots fused_yface parked
-template <int RM, int SOLVER, typename T, int ROWS>
+template <int RM, int SOLVER, typename T, int ROWS, bool WIDE>
 __device__ __forceinline__ uint32_t fused_xface(const RingAcc<RM, ROWS, 0>& ax, const InstDesc& I, const T (&xv)[6],
                                                 bool yneg, flux_t<T, SOLVER> (&F)[NROLE]) {
   constexpr int R = MPR<RM>::R;
@@ -1219,25 +1260,31 @@ __device__ __forceinline__ uint32_t fused_xface(const RingAcc<RM, ROWS, 0>& ax, 
         else px.rhoR = r10;
       }
     }
-    return face_flux<RM, SOLVER, T, 0, true>(ax, &px, I.gamma, I.sigma, F);
+    return face_flux<RM, SOLVER, T, 0, true, WIDE>(ax, &px, I.gamma, I.sigma, F);
   } else {
-    return face_flux<RM, SOLVER, T, 0, false>(ax, (const FacePre<T>*)nullptr, I.gamma, I.sigma, F);
+    return face_flux<RM, SOLVER, T, 0, false, WIDE>(ax, (const FacePre<T>*)nullptr, I.gamma, I.sigma, F);
   }
 }
 
+// The wide form (ROWS = WIDE_ROWS) is for grids that leave the chip idle: tiles
+// of one band of blockDim.y <= WIDE_ROWS warps, each with an SM to itself (168
+// registers per thread, two fields per call of the limiter, no ring).  See
+// stage_wide_rows.
 template <int RM, int SOLVER, typename T, int EP, int ROWS>
-__global__ void __launch_bounds__(32 * ROWS, 16 / ROWS)
+__global__ void __launch_bounds__(32 * ROWS, ROWS == WIDE_ROWS ? 1 : 16 / ROWS)
 k_stage(const InstDesc* __restrict__ insts, int ninst, int ntiles, StageArgs sa) {
   using G = RingGeom<RM, ROWS>;
   constexpr int R = G::R, NS = G::NS, LONG = G::LONG;
   constexpr bool kPre = SOLVER == 5 || SOLVER == 7;
+  constexpr bool WIDE = ROWS == WIDE_ROWS;
   extern __shared__ __align__(128) double smem[];
   __shared__ __align__(8) uint64_t bar;   // completion of the bulk copies of a band's rows
+  const int rows = WIDE ? (int)blockDim.y : ROWS, nthr = 32 * rows;
   double* ring = smem;
-  double* yf = smem + G::RING;
+  double* yf = smem + (WIDE ? (rows + 2 * R + 1) * G::ROWSZ : G::RING);
   const int lane = threadIdx.x, w = threadIdx.y, tid = w * 32 + lane;
   if (tid == 0) {
-    umma::mbar_init(&bar, 32 * ROWS);   // every thread arrives once per bulk fill
+    umma::mbar_init(&bar, nthr);   // every thread arrives once per bulk fill
     umma::mbar_fence_init();
   }
   __syncthreads();
@@ -1253,15 +1300,17 @@ k_stage(const InstDesc* __restrict__ insts, int ninst, int ntiles, StageArgs sa)
     const bool bulk = ring_bulk<RM, ROWS>(I, i0);
     const int sh = i0 - R - ring_col0<R>(i0);   // ring column of grid column i0 - R (0 or 1)
     uint32_t stt = 0;
+    const int jfirst = jseg - 1;   // see below
+    auto slot = [&](int r) { return WIDE ? r - (jfirst - R) : G::slot(r); };
     auto x_acc = [&](int j) {
-      RingAcc<RM, ROWS, 0> a{ring, {G::slot(j) * G::ROWSZ + lane + sh}};
+      RingAcc<RM, ROWS, 0> a{ring, {slot(j) * G::ROWSZ + lane + sh}};
       return a;
     };
     auto y_acc = [&](int j) {
       RingAcc<RM, ROWS, 1> a;
       a.ring = ring;
 #pragma unroll
-      for (int q = 0; q < NS; ++q) a.off[q] = G::slot(j - R + q) * G::ROWSZ + lane + R + sh;
+      for (int q = 0; q < NS; ++q) a.off[q] = slot(j - R + q) * G::ROWSZ + lane + R + sh;
       return a;
     };
     // The bands start one row below the segment: warp 0 of the first band
@@ -1269,12 +1318,12 @@ k_stage(const InstDesc* __restrict__ insts, int ninst, int ntiles, StageArgs sa)
     // jseg - 1 belongs to the segment below and is not updated here), every
     // other warp the y face, the x face and the update of its row.  With
     // seg_rows = 8 nb - 1 the bands are full.
-    const int jfirst = jseg - 1;
-    ring_fill<RM, ROWS>(I, sa, ring, i0, ilast, jfirst - R, min(jfirst + ROWS - 1, jend) + R + 1, tid, bulk, &bar);
+    ring_fill<RM, ROWS>(I, sa, ring, i0, ilast, jfirst - R, min(jfirst + rows - 1, jend) + R + 1, tid, nthr,
+                        jfirst - R, bulk, &bar);
     int band = 0;
-    for (int j0 = jfirst; j0 <= jend; j0 += ROWS, ++band) {
-      const int jl = min(j0 + ROWS - 1, jend);
-      if constexpr (EP != EP_RHS) prefetch_update_rows(I, sa, i0, ilast, max(j0, jseg), jl, tid, 32 * ROWS);
+    for (int j0 = jfirst; j0 <= jend; j0 += rows, ++band) {
+      const int jl = min(j0 + rows - 1, jend);
+      if constexpr (EP != EP_RHS) prefetch_update_rows(I, sa, i0, ilast, max(j0, jseg), jl, tid, nthr);
       // the band's rows have arrived, and every warp has finished the previous
       // band's update (its reads of the face rows that this band overwrites)
       if (bulk) {
@@ -1295,8 +1344,11 @@ k_stage(const InstDesc* __restrict__ insts, int ninst, int ntiles, StageArgs sa)
         __syncthreads();
       }
       // face row k of this band (k = 0 bottom faces, k = w + 1 the faces above row w)
-      const int rb = (band * ROWS) % (ROWS + 1);
-      auto frow = [&](int k) { const int r = k + rb; return yf + (r >= ROWS + 1 ? r - (ROWS + 1) : r) * (NROLE * 32); };
+      const int rb = WIDE ? 0 : (band * ROWS) % (ROWS + 1);
+      auto frow = [&](int k) {
+        const int r = k + rb;
+        return yf + (!WIDE && r >= ROWS + 1 ? r - (ROWS + 1) : r) * (NROLE * 32);
+      };
       const int j = j0 + w;
       const bool face_only = j < jseg;   // warp 0 of the first band
       const bool valid = lane >= 1 && i <= ilast;
@@ -1317,7 +1369,7 @@ k_stage(const InstDesc* __restrict__ insts, int ninst, int ntiles, StageArgs sa)
           T xv[6];
           {
             flux_t<T, SOLVER> Fy[NROLE];
-            stt |= fused_yface<RM, SOLVER, T, ROWS>(ax, y_acc(j), I, kPre ? top : nullptr, yneg, Fy);
+            stt |= fused_yface<RM, SOLVER, T, ROWS, WIDE>(ax, y_acc(j), I, kPre ? top : nullptr, yneg, Fy);
             if constexpr (kPre) {
 #pragma unroll
               for (int c = 0; c < 6; ++c) xv[c] = T(top[c * 32]);
@@ -1325,19 +1377,19 @@ k_stage(const InstDesc* __restrict__ insts, int ninst, int ntiles, StageArgs sa)
 #pragma unroll
             for (int c = 0; c < NROLE; ++c) top[c * 32] = double(Fy[c]);
           }
-          if (!face_only) stt |= fused_xface<RM, SOLVER, T, ROWS>(ax, I, xv, yneg, Fx);
+          if (!face_only) stt |= fused_xface<RM, SOLVER, T, ROWS, WIDE>(ax, I, xv, yneg, Fx);
         }
         // centre values of the point, read before the next band's copies
         // replace the ring rows
-        const double* cen = ring + G::slot(j) * G::ROWSZ + ln + R + sh;
+        const double* cen = ring + slot(j) * G::ROWSZ + ln + R + sh;
         auto cs = [&](int f) { return cen[f * LONG]; };
         cv = Centre{cs(5 + Q_Q), cs(5 + Q_PSI), cs(5 + Q_PHI), cs(5 + Q_EX), cs(5 + Q_EY), cs(5 + Q_EZ),
                     cs(5 + Q_BX), cs(5 + Q_BY), cs(5 + Q_BZ), cs(0), cs(1), cs(2)};
       }
       __syncthreads();   // the band's y fluxes are complete and its ring reads done
-      if (j0 + ROWS <= jend)   // the next band's rows arrive while this band updates
+      if (!WIDE && j0 + ROWS <= jend)   // the next band's rows arrive while this band updates
         ring_fill<RM, ROWS>(I, sa, ring, i0, ilast, j0 + ROWS + R + 1, min(j0 + 2 * ROWS - 1, jend) + R + 1, tid,
-                            bulk, &bar);
+                            nthr, 0, bulk, &bar);
       if (j <= jl && !face_only) {
         double qx[NROLE];
 #pragma unroll
@@ -1369,6 +1421,19 @@ static void launch_tiles(const StageShape& sh, cudaStream_t st, const InstDesc* 
                          cudaEvent_t* ev) {
   using G = FaceGeom<RM, SV, ROWS>;
   const dim3 blk(32, ROWS);
+  if constexpr (kWide<RM, SV> && ROWS == FACE_ROWS) {
+    if (sh.wide_rows && sa.mode == 0) {
+      constexpr int WR = WIDE_ROWS;
+      const size_t bytes = RingGeom<RM, WR>::bytes(sh.wide_rows);
+      const dim3 wblk(32, sh.wide_rows);
+      if (ev) { cudaEventRecord(ev[0], st); cudaEventRecord(ev[1], st); }
+      const int gs = sh.grid[LK_STAGE], ns = sh.ntiles[LK_STAGE];
+      if (sa.l < sa.s) k_stage<RM, SV, T, EP_MID, WR><<<gs, wblk, bytes, st>>>(d, n, ns, sa);
+      else k_stage<RM, SV, T, EP_LAST, WR><<<gs, wblk, bytes, st>>>(d, n, ns, sa);
+      if (ev) cudaEventRecord(ev[2], st);
+      return;
+    }
+  }
   if constexpr (kFused<RM> && ROWS == FACE_ROWS) {
     if (sh.fused && sa.mode == 0) {
       // one launch: ev[0] and ev[1] bracket no work (no separate y-face kernel)
@@ -1402,6 +1467,13 @@ static cudaError_t prepare_tiles() {
     e = cudaFuncSetAttribute(k_xupd<RM, SV, T, EP_MID, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, b0);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_xupd<RM, SV, T, EP_LAST, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, b0);
+  if constexpr (kWide<RM, SV> && ROWS == FACE_ROWS) {
+    const int bw = (int)RingGeom<RM, WIDE_ROWS>::bytes(WIDE_ROWS);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k_stage<RM, SV, T, EP_MID, WIDE_ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, bw);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k_stage<RM, SV, T, EP_LAST, WIDE_ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, bw);
+  }
   if constexpr (kFused<RM> && ROWS == FACE_ROWS) {
     const int bs = (int)RingGeom<RM, ROWS>::bytes();
     if (e == cudaSuccess)
