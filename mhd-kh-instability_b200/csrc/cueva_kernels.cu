@@ -25,6 +25,40 @@ __global__ void k_begin_step(const InstDesc* __restrict__ insts, int ninst, int 
   (void)ninst;
 }
 
+// The 14 primitives of small grids straight from / to the caller's pinned
+// arrays over PCIe: one launch instead of 14 two-dimensional copies of some 6
+// us each (and, going up, instead of the pass of k_begin_step).  32 x 8
+// threads, a warp along a row; bound by PCIe latency and rate (mapped_prims
+// has the times and the size up to which this is the faster way).
+__global__ void __launch_bounds__(256)
+k_upload_begin(const InstDesc* __restrict__ insts, const __grid_constant__ HostPrims h, int cur, int qout,
+               double abt11) {
+  const InstDesc& I = insts[0];
+  const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y;
+  if (i > I.imax || j > I.jmax) return;
+  const long long pc = (long long)j * I.pitch + i, ho = (long long)j * h.pitch + i;
+  double pv[NPRIM];
+#pragma unroll
+  for (int c = 0; c < NPRIM; ++c) pv[c] = h.f[c][ho];
+#pragma unroll
+  for (int c = 0; c < NPRIM; ++c) I.prim[cur][c * I.fstride + pc] = pv[c];
+  begin_step_point(I, abt11, I.aux[cur], I.stage[qout], pc, pv);
+}
+
+__global__ void __launch_bounds__(256)
+k_download(const InstDesc* __restrict__ insts, const __grid_constant__ HostPrims h, int cur, uint32_t* status) {
+  const InstDesc& I = insts[0];
+  const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y;
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0) *status = *I.status;
+  if (i > I.imax || j > I.jmax) return;
+  const long long pc = (long long)j * I.pitch + i, ho = (long long)j * h.pitch + i;
+  double pv[NPRIM];
+#pragma unroll
+  for (int c = 0; c < NPRIM; ++c) pv[c] = I.prim[cur][c * I.fstride + pc];
+#pragma unroll
+  for (int c = 0; c < NPRIM; ++c) h.f[c][ho] = pv[c];
+}
+
 // primitive reconstruction (05_reconstruct.f95:525-746, primitive_rec = 1):
 // per field, the monotonized-central slope along the grid diagonal
 // (limit = 2, funciones.f95:104-147), L = u + x and R = u - x with
@@ -278,6 +312,17 @@ static dim3 point_grid(long long npts, int ninst) {
 cudaError_t launch_begin_step(long long npts, cudaStream_t st, const InstDesc* d, int n, int cur, int qout,
                               double abt11) {
   k_begin_step<<<point_grid(npts, n), 256, 0, st>>>(d, n, cur, qout, abt11);
+  return cudaGetLastError();
+}
+static dim3 row_grid(int imax, int jmax) { return dim3((unsigned)(imax + 32) / 32, (unsigned)(jmax + 8) / 8); }
+cudaError_t launch_upload_begin(cudaStream_t st, const InstDesc* d, int imax, int jmax, const HostPrims& h, int cur,
+                                int qout, double abt11) {
+  k_upload_begin<<<row_grid(imax, jmax), dim3(32, 8), 0, st>>>(d, h, cur, qout, abt11);
+  return cudaGetLastError();
+}
+cudaError_t launch_download(cudaStream_t st, const InstDesc* d, int imax, int jmax, const HostPrims& h, int cur,
+                            uint32_t* status) {
+  k_download<<<row_grid(imax, jmax), dim3(32, 8), 0, st>>>(d, h, cur, status);
   return cudaGetLastError();
 }
 cudaError_t launch_startconvar(long long npts, cudaStream_t st, const InstDesc* d, int n, int cur) {

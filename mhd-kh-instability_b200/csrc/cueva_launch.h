@@ -45,6 +45,19 @@ int stage_wide_rows(int solver, const int* grids, int ngrids, int num_sms);
 // grid rows per fused-stage tile for a grid: a multiple of rows, so that the
 // launch has enough tiles to balance over `slots` resident CTAs
 int stage_seg_rows(int imax, int jmax, int rows, int slots);
+// pinned host arrays as the kernels see them: element (0, 0) of the 14
+// primitive fields, pitch in doubles
+struct HostPrims {
+  double* f[NPRIM];
+  int pitch;
+};
+// small exchanges with the host in one launch each: the 14 fields to
+// prim[cur] with startconvar and stage 1 of them (launch_begin_step's work);
+// prim[cur] to the 14 fields, and the status word to *status
+cudaError_t launch_upload_begin(cudaStream_t st, const InstDesc* d, int imax, int jmax, const HostPrims& h, int cur,
+                                int qout, double abt11);
+cudaError_t launch_download(cudaStream_t st, const InstDesc* d, int imax, int jmax, const HostPrims& h, int cur,
+                            uint32_t* status);
 cudaError_t launch_begin_step(long long npts, cudaStream_t st, const InstDesc* d, int n, int cur, int qout,
                               double abt11);
 cudaError_t launch_startconvar(long long npts, cudaStream_t st, const InstDesc* d, int n, int cur);
