@@ -527,7 +527,7 @@ int32_t cueva_ctx_create(const cueva_params* p, cueva_ctx** out) {
   I.block_count[LK_YFACE] = yface_tiles(c->imax, c->jmax, FACE_ROWS);
   const int grid[2] = {c->imax, c->jmax};
   c->wide_rows = c->shape.wide_rows = stage_wide_rows(p->flux_solver, grid, 1, nsm);
-  I.seg_rows = c->wide_rows ? c->wide_rows - 1 : stage_seg_rows(c->imax, c->jmax, FACE_ROWS, 2 * nsm);
+  I.seg_rows = c->wide_rows ? c->wide_rows - 1 : stage_seg_rows(grid, 1, FACE_ROWS, 2 * nsm);
   I.block_count[LK_STAGE] = stage_tiles(c->imax, c->jmax, I.seg_rows);
   c->shape.rows = FACE_ROWS;
   for (int k : {LK_XUPD, LK_YFACE, LK_STAGE}) {
@@ -1517,12 +1517,13 @@ int32_t ens_apply_shape(cueva_ens* e, int rows, int ctas_per_sm) {
   const int wide = rows == FACE_ROWS && ctas_per_sm == 0
                        ? stage_wide_rows(e->P0.flux_solver, grids.data(), e->n, e->num_sms) : 0;
   e->shape.wide_rows = wide;
+  const int seg = wide ? wide - 1 : stage_seg_rows(grids.data(), e->n, FACE_ROWS, 2 * e->num_sms);
   for (int k = 0; k < e->n; ++k) {
     InstDesc& I = e->I[k];
     I.block_count[LK_XUPD] = xupd_tiles(I.imax, I.jmax, rows);
     I.block_count[LK_YFACE] = yface_tiles(I.imax, I.jmax, rows);
     I.block_count[LK_C2P] = c2p_tiles(I.imax, I.jmax);
-    I.seg_rows = wide ? wide - 1 : stage_seg_rows(I.imax, I.jmax, FACE_ROWS, 2 * e->num_sms);
+    I.seg_rows = seg;
     I.block_count[LK_STAGE] = stage_tiles(I.imax, I.jmax, I.seg_rows);
     for (int t = 0; t < 4; ++t) { I.block_begin[t] = begin[t]; begin[t] += I.block_count[t]; }
   }

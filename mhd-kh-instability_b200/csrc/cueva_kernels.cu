@@ -2,6 +2,11 @@
 // step, routine mirrors) and the dispatch of the stage launches to the
 // per-solver translation units (cueva_stage_{hll,hllc,hlle}.cu; the stage
 // kernels themselves are described in cueva_stage.cuh).
+#include <algorithm>
+#include <functional>
+#include <queue>
+#include <vector>
+
 #include "cueva_launch.h"
 #include "cueva_stage.cuh"
 
@@ -250,19 +255,54 @@ int stage_wide_rows(int solver, const int* grids, int ngrids, int num_sms) {
   return 0;
 }
 
-int stage_seg_rows(int imax, int jmax, int rows, int slots) {
+int stage_seg_rows(const int* grids, int ngrids, int rows, int slots) {
   // A tile of nb bands updates nb * rows - 1 grid rows (its first band also
-  // computes the faces below the segment) and costs about nb band times; the
-  // launch takes about ceil(tiles / slots) tile times.  Pick the band count
-  // with the smallest product (the larger one on ties: fewer repeated faces).
-  const int strips = (imax + 1 + 30) / 31;
+  // computes the faces below the segment) and costs about nb band times.
   int best = 1;
   long long best_cost = -1;
+  if (ngrids == 1) {
+    // One grid: the launch takes about ceil(tiles / slots) tile times.  Pick
+    // the band count with the smallest product (the larger one on ties: fewer
+    // repeated faces).
+    for (int nb = 1; nb <= 32; ++nb) {
+      const long long tiles = stage_tiles(grids[0], grids[1], nb * rows - 1);
+      const long long cost = (tiles + slots - 1) / slots * nb;
+      if (best_cost < 0 || cost <= best_cost) { best_cost = cost; best = nb; }
+    }
+    return best * rows - 1;
+  }
+  // Grids that share a launch share one band count: what counts is how the
+  // tiles of all of them fill the slots, and a count that suits each grid by
+  // itself repeats faces for a balance that the others give anyway.  Hand the
+  // tiles out in launch order, each to the slot that is free first, a tile
+  // taking its bands and 1/20 band to start, and take the count that ends
+  // first.  24 grids of 128 x 64, 256 x 128 and 512 x 256, MP5 HLLC, us a step
+  // for nb = 1..8: 3433 3285 3212 3297 3353 3387 3495 3633; 3 is taken here,
+  // counts of 1, 1 and 3 by each grid's own rule took 3354.
+  constexpr int kBand = 20;
   for (int nb = 1; nb <= 32; ++nb) {
     const int seg = nb * rows - 1;
-    const long long tiles = (long long)strips * ((jmax + 1 + seg - 1) / seg);
-    const long long cost = (tiles + slots - 1) / slots * nb;
-    if (best_cost < 0 || cost <= best_cost) { best_cost = cost; best = nb; }
+    long long tiles = 0, work = 0;
+    for (int k = 0; k < ngrids; ++k) tiles += stage_tiles(grids[2 * k], grids[2 * k + 1], seg);
+    const bool many = tiles > 16LL * slots;   // many waves: the mean and half a tile for the uneven end
+    std::priority_queue<long long, std::vector<long long>, std::greater<long long>> free_at;
+    long long end = 0, longest = 0;
+    for (int k = 0; k < ngrids; ++k) {
+      const int strips = stage_tiles(grids[2 * k], 0, seg), ny = grids[2 * k + 1] + 1;
+      for (int j = 0; j < ny; j += seg) {
+        const long long t = (std::min(seg, ny - j) + rows) / rows * kBand + 1;
+        work += t * strips;
+        longest = std::max(longest, t);
+        for (int s = 0; !many && s < strips; ++s) {
+          long long at = t;
+          if ((int)free_at.size() == slots) { at += free_at.top(); free_at.pop(); }
+          free_at.push(at);
+          end = std::max(end, at);
+        }
+      }
+    }
+    const long long cost = many ? work / slots + longest / 2 : end;
+    if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = nb; }
   }
   return best * rows - 1;
 }

@@ -42,9 +42,10 @@ bool stage_fused_available(int rec_mp, int solver);
 // warps per tile of the fused kernel's wide form for a launch over these grids
 // (pairs of imax, jmax), or 0 where it does not apply
 int stage_wide_rows(int solver, const int* grids, int ngrids, int num_sms);
-// grid rows per fused-stage tile for a grid: a multiple of rows, so that the
-// launch has enough tiles to balance over `slots` resident CTAs
-int stage_seg_rows(int imax, int jmax, int rows, int slots);
+// grid rows per fused-stage tile of a launch over these grids (pairs of imax,
+// jmax): a multiple of rows less one, so that the launch's tiles balance over
+// `slots` resident CTAs
+int stage_seg_rows(const int* grids, int ngrids, int rows, int slots);
 // pinned host arrays as the kernels see them: element (0, 0) of the 14
 // primitive fields, pitch in doubles
 struct HostPrims {
