@@ -3,9 +3,6 @@
 // per-solver translation units (cueva_stage_{hll,hllc,hlle}.cu; the stage
 // kernels themselves are described in cueva_stage.cuh).
 #include <algorithm>
-#include <functional>
-#include <queue>
-#include <vector>
 
 #include "cueva_launch.h"
 #include "cueva_stage.cuh"
@@ -273,35 +270,25 @@ int stage_seg_rows(const int* grids, int ngrids, int rows, int slots) {
   }
   // Grids that share a launch share one band count: what counts is how the
   // tiles of all of them fill the slots, and a count that suits each grid by
-  // itself repeats faces for a balance that the others give anyway.  Hand the
-  // tiles out in launch order, each to the slot that is free first, a tile
-  // taking its bands and 1/20 band to start, and take the count that ends
-  // first.  24 grids of 128 x 64, 256 x 128 and 512 x 256, MP5 HLLC, us a step
-  // for nb = 1..8: 3433 3285 3212 3297 3353 3387 3495 3633; 3 is taken here,
-  // counts of 1, 1 and 3 by each grid's own rule took 3354.
-  constexpr int kBand = 20;
+  // itself repeats faces for a balance that the others give anyway.  With
+  // many unlike tiles the launch takes the mean load of a slot and, for its
+  // uneven end, half of the longest tile; with a slot for every tile, the
+  // longest.  24 grids of 128 x 64, 256 x 128 and 512 x 256, MP5 HLLC: that is
+  // 23.5 22.7 22.5 23.0 23.0 23.5 24.0 24.5 band times for nb = 1..8, measured
+  // 3433 3285 3212 3297 3353 3387 3495 3633 us a step; counts of 1, 1 and 3 by
+  // each grid's own rule took 3354.
   for (int nb = 1; nb <= 32; ++nb) {
     const int seg = nb * rows - 1;
-    long long tiles = 0, work = 0;
-    for (int k = 0; k < ngrids; ++k) tiles += stage_tiles(grids[2 * k], grids[2 * k + 1], seg);
-    const bool many = tiles > 16LL * slots;   // many waves: the mean and half a tile for the uneven end
-    std::priority_queue<long long, std::vector<long long>, std::greater<long long>> free_at;
-    long long end = 0, longest = 0;
+    long long tiles = 0, work = 0, longest = 0;   // in bands
     for (int k = 0; k < ngrids; ++k) {
       const int strips = stage_tiles(grids[2 * k], 0, seg), ny = grids[2 * k + 1] + 1;
-      for (int j = 0; j < ny; j += seg) {
-        const long long t = (std::min(seg, ny - j) + rows) / rows * kBand + 1;
-        work += t * strips;
-        longest = std::max(longest, t);
-        for (int s = 0; !many && s < strips; ++s) {
-          long long at = t;
-          if ((int)free_at.size() == slots) { at += free_at.top(); free_at.pop(); }
-          free_at.push(at);
-          end = std::max(end, at);
-        }
-      }
+      const int full = ny / seg, rest = ny % seg;
+      const int last = rest ? (rest + rows) / rows : 0;
+      tiles += (long long)strips * (full + (rest > 0));
+      work += (long long)strips * (full * nb + last);
+      longest = std::max<long long>(longest, full ? nb : last);
     }
-    const long long cost = many ? work / slots + longest / 2 : end;
+    const long long cost = tiles <= slots ? 2 * slots * longest : 2 * work + slots * longest;
     if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = nb; }
   }
   return best * rows - 1;
