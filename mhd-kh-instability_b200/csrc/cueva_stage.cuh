@@ -778,29 +778,42 @@ __device__ __forceinline__ uint32_t update_point(const InstDesc& I, const StageA
       double acc[NCONS];
 #pragma unroll
       for (int c = 0; c < NCONS; ++c) acc[c] = sa.need_intsum_load ? I.intsum[c * fs + pc] : 0.0;
+      // with Ab = 0 the term ab * F is a zero: the flux of K_m is not read (a
+      // stored K_m may hold its E sources only), which changes at most the sign
+      // of a zero sum.  The stored K_m (m < l) and this stage's K_l have code
+      // of their own: one loop that chose between memory and registers per
+      // field kept more of both alive (k_stage MP5 HLLC: 380 bytes of spills,
+      // now 324).  Steps on a B200: 2048 x 4096 14.39 -> 14.10 ms, 1024 x 2048
+      // 3.93 -> 3.85 ms, mixed MP7 3.73 -> 3.69 ms, 611 x 1003 MP7 900 -> 884 us.
+      // Loading and storing the sums in two groups of fields instead spilled
+      // 490 to 700 bytes: 14.9 to 15.8 ms.
 #pragma unroll 1
-      for (int m = 1; m <= sa.l; ++m) {
+      for (int m = 1; m < sa.l; ++m) {
         const double ab = sa.ab_next[m - 1], abt = sa.abt_next[m - 1];
-        if (ab == 0.0 && abt == 0.0) continue;
-        const double* Km = (m < sa.l) ? I.kbuf + (long long)sa.kslot[m - 1] * NRHS * fs : nullptr;
-        // with Ab = 0 the term ab * F is a zero: the flux of K_m is not read
-        // (a stored K_m may hold its E sources only), which changes at most
-        // the sign of a zero sum
+        const double* Km = I.kbuf + (long long)sa.kslot[m - 1] * NRHS * fs + pc;
+        if (ab != 0.0) {
+#pragma unroll
+          for (int c = 0; c < NCONS; ++c) {
+            if (c >= Q_EX && c <= Q_EZ) acc[c] = acc[c] + (ab * Km[c * fs] - abt * Km[(K_SEX + c - Q_EX) * fs]);
+            else acc[c] = acc[c] + ab * Km[c * fs];
+          }
+        } else if (abt != 0.0) {
+#pragma unroll
+          for (int c = 0; c < NCONS; ++c)
+            if (c >= Q_EX && c <= Q_EZ) acc[c] = acc[c] + (0.0 - abt * Km[(K_SEX + c - Q_EX) * fs]);
+        }
+      }
+      const double ab = sa.ab_next[sa.l - 1], abt = sa.abt_next[sa.l - 1];
+      if (ab != 0.0) {
 #pragma unroll
         for (int c = 0; c < NCONS; ++c) {
-          if (c >= Q_EX && c <= Q_EZ) {
-            const double S = Km ? Km[(K_SEX + c - Q_EX) * fs + pc] : K[K_SEX + c - Q_EX];
-            if (ab == 0.0) {
-              acc[c] = acc[c] + (0.0 - abt * S);
-            } else {
-              const double F = Km ? Km[c * fs + pc] : K[c];
-              acc[c] = acc[c] + (ab * F - abt * S);
-            }
-          } else if (ab != 0.0) {
-            const double F = Km ? Km[c * fs + pc] : K[c];
-            acc[c] = acc[c] + ab * F;
-          }
+          if (c >= Q_EX && c <= Q_EZ) acc[c] = acc[c] + (ab * K[c] - abt * K[K_SEX + c - Q_EX]);
+          else acc[c] = acc[c] + ab * K[c];
         }
+      } else if (abt != 0.0) {
+#pragma unroll
+        for (int c = 0; c < NCONS; ++c)
+          if (c >= Q_EX && c <= Q_EZ) acc[c] = acc[c] + (0.0 - abt * K[K_SEX + c - Q_EX]);
       }
       if (sa.need_intsum_store) {
 #pragma unroll
