@@ -254,41 +254,33 @@ int stage_wide_rows(int solver, const int* grids, int ngrids, int num_sms) {
 
 int stage_seg_rows(const int* grids, int ngrids, int rows, int slots) {
   // A tile of nb bands updates nb * rows - 1 grid rows (its first band also
-  // computes the faces below the segment) and costs about nb band times.
+  // computes the faces below the segment).  Tiles take unlike times (the
+  // limiter's work varies over a flow, and two CTAs share an SM), so a launch
+  // takes the mean load of a slot and, for its uneven end, about half of the
+  // longest tile, whether or not the tiles come out at whole waves.  All grids
+  // of a launch share the band count.  Steps on a B200 (MP5 HLLC where not
+  // said), band count of ceil(tiles / slots) * nb smallest -> this one's:
+  //   300 x 300        5 -> 1   0.367 -> 0.331 ms (MC HLLC 0.308 -> 0.313)
+  //   500 x 1000       8 -> 2   1.192 -> 1.084 ms (MC HLL 0.357 -> 0.359)
+  //   900 x 900       13 -> 2   1.94 -> 1.67 ms
+  //   700 x 1500      15 -> 2   2.24 -> 2.02 ms
+  //   1000 x 2500     18 -> 3   mixed 4.52 -> 4.24 ms, MC 3.05 -> 2.94 ms
+  //   1024 x 2048     10 -> 3   3.87 -> 3.73 ms
+  //   2048 x 4096     13 -> 5   14.19 -> 13.95 ms (4: 14.07, 8: 13.93)
+  //   24 grids of 64 x 128 to 256 x 512: 1, 1 and 3 -> 3, 3.35 -> 3.21 ms
   int best = 1;
   long long best_cost = -1;
-  if (ngrids == 1) {
-    // One grid: the launch takes about ceil(tiles / slots) tile times.  Pick
-    // the band count with the smallest product (the larger one on ties: fewer
-    // repeated faces).
-    for (int nb = 1; nb <= 32; ++nb) {
-      const long long tiles = stage_tiles(grids[0], grids[1], nb * rows - 1);
-      const long long cost = (tiles + slots - 1) / slots * nb;
-      if (best_cost < 0 || cost <= best_cost) { best_cost = cost; best = nb; }
-    }
-    return best * rows - 1;
-  }
-  // Grids that share a launch share one band count: what counts is how the
-  // tiles of all of them fill the slots, and a count that suits each grid by
-  // itself repeats faces for a balance that the others give anyway.  With
-  // many unlike tiles the launch takes the mean load of a slot and, for its
-  // uneven end, half of the longest tile; with a slot for every tile, the
-  // longest.  24 grids of 128 x 64, 256 x 128 and 512 x 256, MP5 HLLC: that is
-  // 23.5 22.7 22.5 23.0 23.0 23.5 24.0 24.5 band times for nb = 1..8, measured
-  // 3433 3285 3212 3297 3353 3387 3495 3633 us a step; counts of 1, 1 and 3 by
-  // each grid's own rule took 3354.
   for (int nb = 1; nb <= 32; ++nb) {
     const int seg = nb * rows - 1;
-    long long tiles = 0, work = 0, longest = 0;   // in bands
+    long long work = 0, longest = 0;   // in bands
     for (int k = 0; k < ngrids; ++k) {
       const int strips = stage_tiles(grids[2 * k], 0, seg), ny = grids[2 * k + 1] + 1;
       const int full = ny / seg, rest = ny % seg;
       const int last = rest ? (rest + rows) / rows : 0;
-      tiles += (long long)strips * (full + (rest > 0));
       work += (long long)strips * (full * nb + last);
       longest = std::max<long long>(longest, full ? nb : last);
     }
-    const long long cost = tiles <= slots ? 2 * slots * longest : 2 * work + slots * longest;
+    const long long cost = 2 * work + slots * longest;
     if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = nb; }
   }
   return best * rows - 1;

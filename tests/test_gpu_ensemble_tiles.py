@@ -1,6 +1,8 @@
-"""Ensembles whose tiles share one segment height (stage_seg_rows over all
-grids): unlike and like grids, ragged strips and segments, few tiles and many
-waves of them, against single runs with each grid's own height, bit for bit."""
+"""Segment heights of the fused stage kernel's tiles (stage_seg_rows).  Grids
+on both sides of the heights of one to four bands against the two-kernel form,
+and ensembles, whose grids share one height -- unlike and like grids, ragged
+strips and segments, few tiles and many waves of them -- against single runs
+with each grid's own height, bit for bit."""
 import numpy as np
 import pytest
 
@@ -51,3 +53,22 @@ def test_shared_segments_equal_single_runs(mix, solver, precision):
             assert np.array_equal(g.interior(n), b[n]), (k, n)
         g.close()
     ens.close()
+
+
+@pytest.mark.parametrize("imax,jmax", [(403, 301), (640, 340), (999, 451), (1003, 777), (1500, 1200), (2200, 1900)])
+@pytest.mark.parametrize("solver,precision", [(7, 0), (7, 1)])
+def test_segments_equal_two_kernels(imax, jmax, solver, precision):
+    from cueva import Cueva
+    prims, out = state(imax, jmax, 0), []
+    for fused in (1, 0):
+        g = Cueva(imax=imax, jmax=jmax, order=2, flux_solver=solver, rec_mp=0, precision=precision, sigma=1e3)
+        g.set_stage_kernel(fused)
+        for n, a in prims.items():
+            g.set_interior(n, a)
+        g.upload()
+        g.step(2)
+        g.download()
+        out.append({n: g.interior(n).copy() for n in prims})
+        g.close()
+    for n in prims:
+        assert np.array_equal(out[0][n], out[1][n]), n
