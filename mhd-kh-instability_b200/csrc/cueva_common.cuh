@@ -128,13 +128,16 @@ template <typename T> __device__ __forceinline__ T fsgn1(T b) { return copysign(
 // advance", IEEE Trans. Computers 53, 2004).  The sign is taken from a, so
 // that signed zeros come out as the division gives them (b > 0, or b's
 // sign).  Exact while nothing under- or overflows on the way: the exponents
-// of b and of every nonzero a are tested, and values out of range take the
-// division itself, in a rolled loop (they are rare, and the code stays small).
+// of b and of every nonzero a are tested (magnitude_key: a subnormal whose
+// high word is zero is no zero), and values out of range take the division
+// itself, in a rolled loop (they are rare, and the code stays small).
 // Used for the 28 flux differences of a point where a spacing is no power of
 // two, and the 14 star-state quotients of an HLLC face.  Steps on a B200,
 // divisions one by one -> shared: 500 x 1000 HLL + MC 433 -> 361 us, 700 x
 // 1500 HLLC + MP9 2.91 -> 2.41 ms, 611 x 1003 HLL + MP7 1214 -> 1001 us, 2048 x
-// 4096 HLLC + MP5 (power-of-two spacings) 16.24 -> 15.43 ms.
+// 4096 HLLC + MP5 (power-of-two spacings) 16.24 -> 15.43 ms.  Telling subnormals
+// from zeros by their low words costs 0.5 to 1 % of a step (13.92 -> 13.99 ms
+// at 2048 x 4096, 359 -> 362 us at 500 x 1000 HLL + MC).
 __device__ __forceinline__ double recip_rn(double b) { return __drcp_rn(b); }
 __device__ __forceinline__ float recip_rn(float b) { return __frcp_rn(b); }
 __device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
@@ -142,6 +145,11 @@ __device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fm
 // sign and exponent bits of a value, and the range of |a| and |b| in them
 __device__ __forceinline__ uint32_t high_word(double x) { return (uint32_t)__double2hiint(x); }
 __device__ __forceinline__ uint32_t high_word(float x) { return __float_as_uint(x); }
+// |x| by its leading bits, zero for zeros alone
+__device__ __forceinline__ uint32_t magnitude_key(double x) {
+  return (high_word(x) & 0x7fffffffu) | min((uint32_t)__double2loint(x), 1u);
+}
+__device__ __forceinline__ uint32_t magnitude_key(float x) { return high_word(x) & 0x7fffffffu; }
 template <typename T> struct DivRange;
 template <> struct DivRange<double> {   // a in 2^-800 .. 2^800, b in 2^-100 .. 2^100
   static constexpr uint32_t a_lo = (1023u - 800u) << 20, a_hi = (1023u + 800u) << 20;
@@ -163,7 +171,7 @@ __device__ __forceinline__ void divide_all(T (&a)[N], T b, T z) {
   uint32_t lo = 0xffffffffu, hi = 0;
 #pragma unroll
   for (int k = 0; k < N; ++k) {
-    const uint32_t h = high_word(a[k]) & 0x7fffffffu;
+    const uint32_t h = magnitude_key(a[k]);
     lo = min(lo, h - 1u);   // a zero passes
     hi = max(hi, h);
   }
