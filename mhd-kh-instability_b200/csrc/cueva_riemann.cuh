@@ -104,7 +104,8 @@ __device__ __forceinline__ Phys<T> physical(const Side<T>& s, T gamma, T W) {
   const T En = X::En(s), Et1 = X::Et1(s), Et2 = X::Et2(s);
   const T Bn = X::Bn(s), Bt1 = X::Bt1(s), Bt2 = X::Bt2(s);
   f.Ftau = (Bt2 * Et1 - Bt1 * Et2) + hW2 * vn;
-  const T FSn = fma_rn(T(0.5), E2B2, -pw2(En) - pw2(Bn) + hW2 * pw2(vn));   // half of E2B2 is exact
+  // half of E2B2 is exact, or subnormal and lost beside the pressure
+  const T FSn = fma_rn(T(0.5), E2B2, -pw2(En) - pw2(Bn) + hW2 * pw2(vn));
   if constexpr (PS) f.FSn = FSn + s.dp;
   else f.FSn = FSn + s.p;
   f.FSt1 = -En * Et1 - Bn * Bt1 + hW2 * vn * vt1;
@@ -373,7 +374,8 @@ __device__ __forceinline__ void hllc_fluxes(const Side<T>& L, const Side<T>& R, 
   // tau, S receive the star correction; E, B, q keep the HLL fluxes.
   if (V > T(0.0) || V < T(0.0)) {
     const T k = V > T(0.0) ? omV : opV;
-    auto star = [&](T f, T r, T l) { return fma_rn(k * (r - l), h, f); };   // f + (k (r - l)) / 2
+    // (an FMA would be exact but for subnormal halves, which a decaying psi or phi reaches)
+    auto star = [&](T f, T r, T l) { return f + k * (r - l) * h; };
     A[R_PSI] = star(psi_f, psiR, psiL);
     A[R_PHI] = star(phi_f, phiR, phiL);
     A[R_D] = star(D_f, DR, DL);
@@ -581,7 +583,8 @@ __device__ __forceinline__ void hllcmc_fluxes(const Side<T>& L, const Side<T>& R
   // v* == 0 the HLL fluxes; E, B and q keep the HLL fluxes throughout
   if (V > T(0.0) || V < T(0.0)) {
     const T k = V > T(0.0) ? omV : opV;
-    auto star = [&](T f, T r, T l) { return fma_rn(k * (r - l), h, f); };   // f + (k (r - l)) / 2
+    // (an FMA would be exact but for subnormal halves, which a decaying psi or phi reaches)
+    auto star = [&](T f, T r, T l) { return f + k * (r - l) * h; };
     A[R_PSI] = star(psi_f, psiR, psiL);
     A[R_PHI] = star(phi_f, phiR, phiL);
     A[R_D] = star(D_f, DR, DL);
