@@ -142,8 +142,10 @@ int32_t cueva_download(cueva_ctx* ctx, uint32_t groups);
  * caller must not read, modify, rebind or free them (later calls such as
  * cueva_step only order their device work after the copies; they do not
  * wait).  A following cueva_upload of the same arrays waits per field on the
- * device, so field f goes back up while field f+1 still comes down.  Kernel
- * status is reported by the next call that synchronises. */
+ * device, so field f goes back up while field f+1 still comes down (pinned
+ * primitives of up to 4 MB in all go up in one launch after the whole
+ * readback, which is faster at that size).  Kernel status is reported by the
+ * next call that synchronises. */
 int32_t cueva_download_async(cueva_ctx* ctx, uint32_t groups);
 
 /* ---- the hot path ----------------------------------------------------- */

@@ -365,11 +365,17 @@ bool host_mapped(const void* p, size_t bytes, void** dev) {
 // 64 x 32 (0.24 MB) 98 / 66 -> 29 / 24 us, 256 x 128 (3.7 MB) 198 / 130 -> 116 / 95,
 // 400 x 200 (9 MB) 294 / 223 -> 236 / 203, but 512 x 256 (15 MB) 397 / 325 -> 377 /
 // 341 and 1024 x 512 (59 MB) 1203 / 1113 -> 1411 / 1450.
+// With an asynchronous readback pending the launch has to wait for all of it,
+// while a copy waits for its own field's: there the limit is lower.  Loop of
+// upload, one step (MP5 HLLC, SSP2) and asynchronous download, copies / one
+// launch: 64 x 32 167 / 134 us, 256 x 128 (3.7 MB) 284 / 278, but 300 x 150
+// (5.1 MB) 322 / 337, 300 x 250 (8.5 MB) 535 / 562, 420 x 205 (9.7 MB) 585 / 620.
 constexpr size_t kMappedBytes = size_t(10) << 20;
+constexpr size_t kMappedPendingBytes = size_t(4) << 20;
 
 bool mapped_prims(cueva_ctx* c, HostPrims& h) {
   const size_t npt = (size_t)c->nx * c->ny;
-  if (npt * NPRIM * sizeof(double) > kMappedBytes) return false;
+  if (npt * NPRIM * sizeof(double) > (c->dl_pending ? kMappedPendingBytes : kMappedBytes)) return false;
   h.pitch = c->imax + 13;
   const size_t span = ((size_t)(c->ny - 1) * h.pitch + c->nx) * sizeof(double);   // first to last interior element
   for (int f = 0; f < NPRIM; ++f) {
