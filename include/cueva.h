@@ -162,7 +162,11 @@ int32_t cueva_step(cueva_ctx* ctx, int32_t nsteps);
  * memory); fused = 0 as a y-face kernel and an x-face + update kernel that
  * pass the y fluxes through device memory.  Both give bit-identical results.
  * The default is 1 where the fused kernel exists (MP5 and the MC slopes of
- * flux routines 1-4); elsewhere 1 is refused with CUEVA_ERR_ARG. */
+ * flux routines 1-4); elsewhere 1 is refused with CUEVA_ERR_ARG.  Grids whose
+ * one-band tiles find an SM each (flux routines 5-7, about 250 x 200 points)
+ * run one kernel per stage for every reconstruction until 0 is set:
+ * cueva_get_stage_kernel answers 0 for MP7 and MP9 there, too, and what 0 sets
+ * aside for them stays so for the life of the context. */
 int32_t cueva_set_stage_kernel(cueva_ctx* ctx, int32_t fused);
 /* bytes of the context's device field slab (state, stage sums, stored stage
  * right-hand sides, flux scratch); no counterpart in the reference */

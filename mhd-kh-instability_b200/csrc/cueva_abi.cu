@@ -594,8 +594,7 @@ int32_t cueva_set_stage_kernel(cueva_ctx* c, int32_t fused) {
   CUDA_TRY(cudaStreamSynchronize(c->stream));
   destroy_graphs(c);
   c->shape.fused = fused != 0;
-  // the two-kernel form on request; MP7 and MP9 have no fused form to choose and keep theirs
-  if (stage_fused_available(c->P.rec_mp, c->P.flux_solver)) c->shape.wide_rows = fused ? c->wide_rows : 0;
+  c->shape.wide_rows = fused ? c->wide_rows : 0;
   return CUEVA_OK;
 }
 
