@@ -409,9 +409,10 @@ __global__ void k_round(int n, const float* w, float* wr) {
   if (i < n) wr[i] = __bfloat162float(__float2bfloat16(w[i]));
 }
 
-// one state of the batch con2prim arrays
-__device__ __forceinline__ C2PIn batch_state(long long n, long long i, const double* __restrict__ cons,
-                                             const double* __restrict__ prev) {
+// one state of the batch con2prim arrays.  No array of the batch kernels is
+// __restrict__: a caller may recover in place (out = prev, seeds = its
+// pressures), and a state is read whole before it is written.
+__device__ __forceinline__ C2PIn batch_state(long long n, long long i, const double* cons, const double* prev) {
   return C2PIn{cons[i], cons[n + i], cons[2 * n + i], cons[3 * n + i], cons[4 * n + i], cons[5 * n + i],
                cons[6 * n + i], cons[7 * n + i], cons[8 * n + i], cons[9 * n + i], cons[10 * n + i],
                prev[2 * n + i], prev[3 * n + i], prev[4 * n + i], prev[i], prev[n + i]};
@@ -428,8 +429,8 @@ __device__ __forceinline__ void batch_recover(long long n, long long i, const C2
 
 // batch con2prim without the network: method 1 Cardano (iters 0), 3 Newton
 // from seed[i]
-__global__ void k_c2p_batch(long long n, int method, double gamma, double eps1, const double* __restrict__ cons,
-                            const double* __restrict__ prev, const double* __restrict__ seed, double* out, int* iters) {
+__global__ void k_c2p_batch(long long n, int method, double gamma, double eps1, const double* cons,
+                            const double* prev, const double* seed, double* out, int* iters) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const C2PIn in = batch_state(n, i, cons, prev);
     if (method == 1) {
@@ -522,7 +523,7 @@ __device__ __forceinline__ void c2p_layer(float* act, const float* wt, const flo
 
 __global__ void __launch_bounds__(CN_ROWS, 3)
 k_c2p_network(long long n, int method, double gamma, double eps1, const MLPDevice* __restrict__ M,
-              const double* __restrict__ cons, const double* __restrict__ prev, double* out, int* iters) {
+              const double* cons, const double* prev, double* out, int* iters) {
   extern __shared__ __align__(16) unsigned char cn_smem[];
   C2PNet& S = *reinterpret_cast<C2PNet*>(cn_smem);
   const int t = threadIdx.x;
