@@ -542,7 +542,7 @@ int32_t cueva_ctx_create(const cueva_params* p, cueva_ctx** out) {
   }
   // the fused stage kernel where it exists (k_yface + k_xupd otherwise)
   c->shape.fused = stage_fused_available(p->rec_mp, p->flux_solver);
-  if (prepare_stage(p->rec_mp, p->flux_solver, p->precision) != cudaSuccess ||
+  if (prepare_stage(p->rec_mp, p->flux_solver, p->precision, c->wide_rows != 0) != cudaSuccess ||
       cudaMemcpy(c->d_inst, &I, sizeof(InstDesc), cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking) != cudaSuccess) {
     cueva_ctx_destroy(c); cudaGetLastError();
@@ -1401,7 +1401,7 @@ int32_t cueva_flux_rhs_noalloc(const cueva_params* p, const double* prim, const 
       CUDA_TRY(cudaGetSymbolAddress(&b, g_noalloc_scratch));
       for (int rm = 0; rm < 3; ++rm)
         for (int sv : {5, 6, 7})
-          for (int pr = 0; pr < 2; ++pr) CUDA_TRY(prepare_stage(rm, sv, pr));
+          for (int pr = 0; pr < 2; ++pr) CUDA_TRY(prepare_stage(rm, sv, pr, false));
       g_noalloc_base[p->device] = b;
     }
     base = (char*)g_noalloc_base[p->device];
@@ -1514,13 +1514,24 @@ void ens_destroy_graphs(cueva_ens* e) {
       if (g) { cudaGraphExecDestroy(g); g = nullptr; }
 }
 
+// (imax, jmax) of the instances
+std::vector<int> ens_grids(const cueva_ens* e) {
+  std::vector<int> grids;
+  for (const InstDesc& I : e->I) { grids.push_back(I.imax); grids.push_back(I.jmax); }
+  return grids;
+}
+
+// warps per tile of the wide form for a tile height and CTA count per SM, or 0
+int ens_wide_rows(const cueva_ens* e, int rows, int ctas_per_sm) {
+  if (rows != FACE_ROWS || ctas_per_sm != 0) return 0;
+  return stage_wide_rows(e->P0.flux_solver, ens_grids(e).data(), e->n, e->num_sms);
+}
+
 // tile ranges for a tile height and the launch grid for a CTA count per SM
 int32_t ens_apply_shape(cueva_ens* e, int rows, int ctas_per_sm) {
   int begin[4] = {0, 0, 0, 0};
-  std::vector<int> grids;
-  for (const InstDesc& I : e->I) { grids.push_back(I.imax); grids.push_back(I.jmax); }
-  const int wide = rows == FACE_ROWS && ctas_per_sm == 0
-                       ? stage_wide_rows(e->P0.flux_solver, grids.data(), e->n, e->num_sms) : 0;
+  const std::vector<int> grids = ens_grids(e);
+  const int wide = ens_wide_rows(e, rows, ctas_per_sm);
   e->shape.wide_rows = wide;
   const int seg = wide ? wide - 1 : stage_seg_rows(grids.data(), e->n, FACE_ROWS, 2 * e->num_sms);
   for (int k = 0; k < e->n; ++k) {
@@ -1643,7 +1654,8 @@ int32_t cueva_ens_create(const cueva_params* params, int32_t n, cueva_ens** out)
       if (pts > e->max_points) e->max_points = pts;
     }
   }
-  if (ce == cudaSuccess && prepare_stage(e->P0.rec_mp, e->P0.flux_solver, e->P0.precision) != cudaSuccess)
+  if (ce == cudaSuccess && prepare_stage(e->P0.rec_mp, e->P0.flux_solver, e->P0.precision,
+                                         ens_wide_rows(e, FACE_ROWS, 0) != 0) != cudaSuccess)
     ce = cudaErrorInvalidValue;
   if (ce == cudaSuccess) ce = cudaStreamCreateWithFlags(&e->own_stream, cudaStreamNonBlocking);
   if (ce != cudaSuccess) {

@@ -286,9 +286,9 @@ int stage_seg_rows(const int* grids, int ngrids, int rows, int slots) {
   return best * rows - 1;
 }
 
-cudaError_t prepare_stage(int rec_mp, int solver, int prec) {
+cudaError_t prepare_stage(int rec_mp, int solver, int prec, bool wide) {
 #define CUEVA_PREPARE_CASE(K, NAME) \
-  case K: return prec ? prepare_stage_##NAME##_mixed(rec_mp) : prepare_stage_##NAME##_fp64(rec_mp);
+  case K: return prec ? prepare_stage_##NAME##_mixed(rec_mp, wide) : prepare_stage_##NAME##_fp64(rec_mp, wide);
   switch (solver) {
     CUEVA_PREPARE_CASE(1, lax)
     CUEVA_PREPARE_CASE(2, mcl)

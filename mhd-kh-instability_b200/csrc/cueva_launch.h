@@ -16,12 +16,13 @@ struct MLPDevice;
 int32_t mlp_device_image(const cueva_mlp* M, MLPDevice* out);
 int mlp_device_of(const cueva_mlp* M);
 // sets the shared-memory limits of the stage kernels (call once per device
-// before the first launch or capture)
-cudaError_t prepare_stage(int rec_mp, int solver, int prec);
+// before the first launch or capture), which also loads their code: those of
+// the wide form only where wide is set, for grids that run it
+cudaError_t prepare_stage(int rec_mp, int solver, int prec, bool wide);
 // per-solver, per-precision halves of prepare_stage / launch_stage
 // (cueva_stage_*.cu; _fp64 plain FP64, _mixed the mixed-precision kernels)
 #define CUEVA_DECLARE_STAGE_UNIT(NAME, P)                                                                   \
-  cudaError_t prepare_stage_##NAME##_##P(int rec_mp);                                                       \
+  cudaError_t prepare_stage_##NAME##_##P(int rec_mp, bool wide);                                            \
   cudaError_t launch_stage_##NAME##_##P(int rec_mp, const StageShape& sh, cudaStream_t st, const InstDesc* d, \
                                         int n, const StageArgs& sa, cudaEvent_t* ev);
 #define CUEVA_DECLARE_STAGE_SOLVER(NAME) CUEVA_DECLARE_STAGE_UNIT(NAME, fp64) CUEVA_DECLARE_STAGE_UNIT(NAME, mixed)

@@ -1470,7 +1470,7 @@ static void launch_tiles(const StageShape& sh, cudaStream_t st, const InstDesc* 
 }
 
 template <int RM, int SV, typename T, int ROWS>
-static cudaError_t prepare_tiles() {
+static cudaError_t prepare_tiles(bool wide) {
   using G = FaceGeom<RM, SV, ROWS>;
   const int b0 = (int)G::bytes(0), b1 = (int)G::bytes(1);
   cudaError_t e = cudaFuncSetAttribute(k_yface<RM, SV, T, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, b1);
@@ -1482,9 +1482,9 @@ static cudaError_t prepare_tiles() {
     e = cudaFuncSetAttribute(k_xupd<RM, SV, T, EP_LAST, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, b0);
   if constexpr (kWide<RM, SV> && ROWS == FACE_ROWS) {
     const int bw = (int)RingGeom<RM, WIDE_ROWS>::bytes(WIDE_ROWS);
-    if (e == cudaSuccess)
+    if (wide && e == cudaSuccess)
       e = cudaFuncSetAttribute(k_stage<RM, SV, T, EP_MID, WIDE_ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, bw);
-    if (e == cudaSuccess)
+    if (wide && e == cudaSuccess)
       e = cudaFuncSetAttribute(k_stage<RM, SV, T, EP_LAST, WIDE_ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, bw);
   }
   if constexpr (kFused<RM> && ROWS == FACE_ROWS) {
@@ -1505,9 +1505,9 @@ static void launch_rm_sv(const StageShape& sh, cudaStream_t st, const InstDesc* 
 }
 
 template <int RM, int SV, typename T>
-static cudaError_t prepare_rm_sv() {
-  cudaError_t e = prepare_tiles<RM, SV, T, 8>();
-  if (e == cudaSuccess) e = prepare_tiles<RM, SV, T, 4>();
+static cudaError_t prepare_rm_sv(bool wide) {
+  cudaError_t e = prepare_tiles<RM, SV, T, 8>(wide);
+  if (e == cudaSuccess) e = prepare_tiles<RM, SV, T, 4>(wide);
   return e;
 }
 
@@ -1532,14 +1532,14 @@ cudaError_t launch_stage_solver(int rec_mp, const StageShape& sh, cudaStream_t s
 }
 
 template <int SV, typename T>
-cudaError_t prepare_stage_solver(int rec_mp) {
+cudaError_t prepare_stage_solver(int rec_mp, bool wide) {
   if constexpr (SV >= 1 && SV <= 4) {
-    return prepare_rm_sv<3, SV, T>();
+    return prepare_rm_sv<3, SV, T>(wide);
   } else {
     switch (rec_mp) {
-      case 0: return prepare_rm_sv<0, SV, T>();
-      case 1: return prepare_rm_sv<1, SV, T>();
-      case 2: return prepare_rm_sv<2, SV, T>();
+      case 0: return prepare_rm_sv<0, SV, T>(wide);
+      case 1: return prepare_rm_sv<1, SV, T>(wide);
+      case 2: return prepare_rm_sv<2, SV, T>(wide);
       default: return cudaErrorInvalidValue;
     }
   }
@@ -1554,14 +1554,18 @@ cudaError_t prepare_stage_solver(int rec_mp) {
                                           int n, const StageArgs& sa, cudaEvent_t* ev) {                       \
     return launch_stage_solver<SV, float>(rec_mp, sh, st, d, n, sa, ev);                                       \
   }                                                                                                            \
-  cudaError_t prepare_stage_##NAME##_mixed(int rec_mp) { return prepare_stage_solver<SV, float>(rec_mp); }
+  cudaError_t prepare_stage_##NAME##_mixed(int rec_mp, bool wide) {                                            \
+    return prepare_stage_solver<SV, float>(rec_mp, wide);                                                      \
+  }
 #else
 #define CUEVA_STAGE_UNIT(NAME, SV)                                                                             \
   cudaError_t launch_stage_##NAME##_fp64(int rec_mp, const StageShape& sh, cudaStream_t st, const InstDesc* d, \
                                          int n, const StageArgs& sa, cudaEvent_t* ev) {                       \
     return launch_stage_solver<SV, double>(rec_mp, sh, st, d, n, sa, ev);                                     \
   }                                                                                                           \
-  cudaError_t prepare_stage_##NAME##_fp64(int rec_mp) { return prepare_stage_solver<SV, double>(rec_mp); }
+  cudaError_t prepare_stage_##NAME##_fp64(int rec_mp, bool wide) {                                            \
+    return prepare_stage_solver<SV, double>(rec_mp, wide);                                                    \
+  }
 #endif
 
 }  // namespace cueva
