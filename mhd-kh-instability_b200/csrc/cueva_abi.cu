@@ -8,6 +8,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -223,6 +224,83 @@ void fill_desc(const cueva_params* p, const InstGeom& G, int nkslot, double* sla
   I.block_count[LK_C2P] = c2p_tiles(G.imax, G.jmax);
 }
 
+// Pinned words that status read-backs land in.  Page-locking costs 1 to 2.7 ms
+// and 0.4 ms to undo on a B200 host (a small context is otherwise created in
+// 0.8 ms), so the contexts of a device share one page of words: taken at
+// creation, given back at destruction, the page (4 KB) kept for the next
+// context.  A page is known by its buffer id: after a device reset the id is
+// gone, and a new page takes its place.  p is null where no word is left (or
+// none can be had): the read-back then goes through pageable memory.
+struct StatusWord {
+  uint32_t* p = nullptr;
+  unsigned long long page = 0;   // buffer id
+};
+struct StatusPage {
+  uint32_t* words = nullptr;
+  unsigned long long id = 0;
+  std::vector<uint32_t*> spare;
+};
+constexpr size_t kStatusWords = 1024;
+std::mutex g_status_mu;
+std::map<int, StatusPage>& g_status_pages = *new std::map<int, StatusPage>;   // by device; contexts may outlive statics
+
+// attributes of a host or device pointer (the driver's; null if it has none)
+PFN_cuPointerGetAttributes pointer_query() {
+  static const PFN_cuPointerGetAttributes query = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult r;
+    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &fn, 7000, cudaEnableDefault, &r) != cudaSuccess ||
+        r != cudaDriverEntryPointSuccess)
+      fn = nullptr;
+    return (PFN_cuPointerGetAttributes)fn;
+  }();
+  return query;
+}
+
+// process-wide unique id of the allocation that holds p, 0 if none does
+unsigned long long buffer_id(const void* p) {
+  CUpointer_attribute what[2] = {CU_POINTER_ATTRIBUTE_BUFFER_ID, CU_POINTER_ATTRIBUTE_MEMORY_TYPE};
+  unsigned long long id = 0;
+  unsigned type = 0;
+  void* out[2] = {&id, &type};
+  if (!pointer_query() || pointer_query()(2, what, out, (CUdeviceptr)p) != CUDA_SUCCESS || type != CU_MEMORYTYPE_HOST)
+    return 0;
+  return id;
+}
+
+// a word of the current device dev
+StatusWord acquire_status_word(int dev) {
+  std::lock_guard<std::mutex> lock(g_status_mu);
+  StatusPage& page = g_status_pages[dev];
+  if (page.words && buffer_id(page.words) != page.id) page = StatusPage();
+  if (!page.words) {
+    uint32_t* words = nullptr;
+    if (cudaHostAlloc(&words, kStatusWords * sizeof(uint32_t), cudaHostAllocDefault) != cudaSuccess) {
+      cudaGetLastError();
+      return {};
+    }
+    const unsigned long long id = buffer_id(words);
+    if (!id) {
+      cudaFreeHost(words);
+      return {};
+    }
+    page.words = words;
+    page.id = id;
+    for (size_t k = kStatusWords; k-- > 0;) page.spare.push_back(words + k);
+  }
+  if (page.spare.empty()) return {};
+  StatusWord w{page.spare.back(), page.id};
+  page.spare.pop_back();
+  return w;
+}
+
+void release_status_word(int dev, const StatusWord& w) {
+  if (!w.p) return;
+  std::lock_guard<std::mutex> lock(g_status_mu);
+  StatusPage& page = g_status_pages[dev];
+  if (page.words && page.id == w.page) page.spare.push_back(w.p);
+}
+
 }  // namespace
 
 struct cueva_ctx {
@@ -236,7 +314,7 @@ struct cueva_ctx {
   // device memory
   double* slab = nullptr;
   uint32_t* d_status = nullptr;
-  uint32_t* h_status = nullptr;   // pinned: where the status word is read back to
+  StatusWord h_status;    // pinned: where the status word is read back to
   unsigned long long* d_counters = nullptr;
   InstDesc* d_inst = nullptr;
   InstDesc h_inst{};
@@ -315,10 +393,10 @@ double* prim_f(cueva_ctx* c, int buf, int f) { return c->h_inst.prim[buf] + (lon
 double* aux_f(cueva_ctx* c, int buf, int f) { return c->h_inst.aux[buf] + (long long)f * c->fstride; }
 double* stage_f(cueva_ctx* c, int buf, int f) { return c->h_inst.stage[buf] + (long long)f * c->fstride; }
 
-// waits for the stream and reports the status word that h_status received
-int32_t finish_status(cueva_ctx* c) {
+// waits for the stream and reports the status word that *word received
+int32_t finish_status(cueva_ctx* c, const uint32_t* word) {
   CUDA_TRY(cudaStreamSynchronize(c->stream));
-  const uint32_t st = *(volatile uint32_t*)c->h_status;
+  const uint32_t st = *(const volatile uint32_t*)word;
   if (st) {
     char buf[160];
     snprintf(buf, sizeof buf, "kernel status 0x%x (1 con2prim, 2 superluminal, 4 hllc_vel, 8 v* not finite, 16 non-finite state, 32 HLLE wave speed, 64 tensor-core wait, 128 tensor-core teardown: context suspect, 256 stencil copy wait)", st);
@@ -327,22 +405,17 @@ int32_t finish_status(cueva_ctx* c) {
   return CUEVA_OK;
 }
 int32_t read_status(cueva_ctx* c) {
-  CUDA_TRY(cudaMemcpyAsync(c->h_status, c->d_status, 4, cudaMemcpyDeviceToHost, c->stream));
-  return finish_status(c);
+  uint32_t st = 0;
+  uint32_t* word = c->h_status.p ? c->h_status.p : &st;
+  CUDA_TRY(cudaMemcpyAsync(word, c->d_status, 4, cudaMemcpyDeviceToHost, c->stream));
+  return finish_status(c, word);
 }
 
 // Whether the kernels can reach the host memory at [p, p + bytes): one pinned
 // range that the device maps.  *dev: its address there.  The range is asked
 // for at every call (nothing is remembered about an address).
 bool host_mapped(const void* p, size_t bytes, void** dev) {
-  static const PFN_cuPointerGetAttributes query = [] {
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult r;
-    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &fn, 7000, cudaEnableDefault, &r) != cudaSuccess ||
-        r != cudaDriverEntryPointSuccess)
-      fn = nullptr;
-    return (PFN_cuPointerGetAttributes)fn;
-  }();
+  const PFN_cuPointerGetAttributes query = pointer_query();
   if (!query || (uintptr_t)p % sizeof(double) != 0) return false;
   CUpointer_attribute what[4] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
                                  CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
@@ -516,11 +589,11 @@ int32_t cueva_ctx_create(const cueva_params* p, cueva_ctx** out) {
   }
   cudaMemset(c->slab, 0, (size_t)G.nslab * sizeof(double));
   if (cudaMalloc(&c->d_status, 4) != cudaSuccess || cudaMalloc(&c->d_counters, 3 * 8) != cudaSuccess ||
-      cudaMalloc(&c->d_inst, sizeof(InstDesc)) != cudaSuccess ||
-      cudaHostAlloc(&c->h_status, sizeof(uint32_t), cudaHostAllocDefault) != cudaSuccess) {
+      cudaMalloc(&c->d_inst, sizeof(InstDesc)) != cudaSuccess) {
     cueva_ctx_destroy(c); cudaGetLastError();
     return fail(CUEVA_ERR_CUDA, "cudaMalloc of the context descriptors failed");
   }
+  c->h_status = acquire_status_word(c->dev);
   cudaMemset(c->d_status, 0, 4);
   cudaMemset(c->d_counters, 0, 24);
   InstDesc& I = c->h_inst;
@@ -560,7 +633,7 @@ int32_t cueva_ctx_destroy(cueva_ctx* c) {
   destroy_graphs(c);
   if (c->slab) cudaFree(c->slab);
   if (c->d_status) cudaFree(c->d_status);
-  if (c->h_status) cudaFreeHost(c->h_status);
+  release_status_word(c->dev, c->h_status);
   if (c->d_counters) cudaFree(c->d_counters);
   if (c->d_inst) cudaFree(c->d_inst);
   if (c->d_mlp) cudaFree(c->d_mlp);
@@ -684,9 +757,9 @@ int32_t cueva_download(cueva_ctx* c, uint32_t groups) {
   if (int32_t e = check_ctx(c)) return e;
   CUDA_TRY(cudaSetDevice(c->dev));
   HostPrims h;
-  if (groups == CUEVA_G_PRIMS && mapped_prims(c, h)) {
-    CUDA_TRY(launch_download(c->stream, c->d_inst, c->imax, c->jmax, h, c->cur, c->h_status));
-    return finish_status(c);
+  if (groups == CUEVA_G_PRIMS && c->h_status.p && mapped_prims(c, h)) {
+    CUDA_TRY(launch_download(c->stream, c->d_inst, c->imax, c->jmax, h, c->cur, c->h_status.p));
+    return finish_status(c, c->h_status.p);
   }
   if (groups & CUEVA_G_PRIMS)
     for (int f = 0; f < NPRIM; ++f)
