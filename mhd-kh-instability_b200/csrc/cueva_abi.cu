@@ -606,7 +606,7 @@ int32_t cueva_ctx_create(const cueva_params* p, cueva_ctx** out) {
   I.block_count[LK_YFACE] = yface_tiles(c->imax, c->jmax, FACE_ROWS);
   const int grid[2] = {c->imax, c->jmax};
   c->wide_rows = c->shape.wide_rows = stage_wide_rows(p->flux_solver, grid, 1, nsm);
-  I.seg_rows = c->wide_rows ? c->wide_rows - 1 : stage_seg_rows(grid, 1, FACE_ROWS, 2 * nsm);
+  I.seg_rows = c->wide_rows ? c->wide_rows - 1 : stage_seg_rows(grid, 1, FACE_ROWS, 2 * nsm, p->flux_solver <= 4);
   I.block_count[LK_STAGE] = stage_tiles(c->imax, c->jmax, I.seg_rows);
   c->shape.rows = FACE_ROWS;
   for (int k : {LK_XUPD, LK_YFACE, LK_STAGE}) {
@@ -1606,7 +1606,8 @@ int32_t ens_apply_shape(cueva_ens* e, int rows, int ctas_per_sm) {
   const std::vector<int> grids = ens_grids(e);
   const int wide = ens_wide_rows(e, rows, ctas_per_sm);
   e->shape.wide_rows = wide;
-  const int seg = wide ? wide - 1 : stage_seg_rows(grids.data(), e->n, FACE_ROWS, 2 * e->num_sms);
+  const int seg = wide ? wide - 1 : stage_seg_rows(grids.data(), e->n, FACE_ROWS, 2 * e->num_sms,
+                                                     e->P0.flux_solver <= 4);
   for (int k = 0; k < e->n; ++k) {
     InstDesc& I = e->I[k];
     I.block_count[LK_XUPD] = xupd_tiles(I.imax, I.jmax, rows);

@@ -252,24 +252,34 @@ int stage_wide_rows(int solver, const int* grids, int ngrids, int num_sms) {
   return 0;
 }
 
-int stage_seg_rows(const int* grids, int ngrids, int rows, int slots) {
+int stage_seg_rows(const int* grids, int ngrids, int rows, int slots, bool even) {
   // A tile of nb bands updates nb * rows - 1 grid rows (its first band also
-  // computes the faces below the segment).  Tiles take unlike times (the
-  // limiter's work varies over a flow, and two CTAs share an SM), so a launch
-  // takes the mean load of a slot and, for its uneven end, about half of the
-  // longest tile, whether or not the tiles come out at whole waves.  All grids
-  // of a launch share the band count.  Steps on a B200 (MP5 HLLC where not
-  // said), band count of ceil(tiles / slots) * nb smallest -> this one's:
-  //   300 x 300        5 -> 1   0.367 -> 0.331 ms (MC HLLC 0.308 -> 0.313)
-  //   500 x 1000       8 -> 2   1.192 -> 1.084 ms (MC HLL 0.357 -> 0.359)
-  //   900 x 900       13 -> 2   1.94 -> 1.67 ms
-  //   700 x 1500      15 -> 2   2.24 -> 2.02 ms
-  //   1000 x 2500     18 -> 3   mixed 4.52 -> 4.24 ms, MC 3.05 -> 2.94 ms
-  //   1024 x 2048     10 -> 3   3.87 -> 3.73 ms
-  //   2048 x 4096     13 -> 5   14.19 -> 13.95 ms (4: 14.07, 8: 13.93)
-  //   24 grids of 64 x 128 to 256 x 512: 1, 1 and 3 -> 3, 3.35 -> 3.21 ms
+  // computes the faces below the segment).  All grids of a launch share the
+  // band count.  Two models of a launch's time, in band times:
+  //   mean   tiles take unlike times (the limiter's work varies over a flow,
+  //          and two CTAs share an SM): the mean load of a slot and, for the
+  //          uneven end, about half of the longest tile;
+  //   waves  tiles take their bands: whole waves of full tiles, the short
+  //          tiles of the last rows on the slots left idle.
+  // Ensembles have unlike tiles by construction and take the mean.  A single
+  // grid's time lies between the two, nearer to the mean the more its tiles
+  // differ and the more waves there are; `even` (the MC routines: no limiter)
+  // with less than three waves of one-band tiles goes by the waves.  A tile's
+  // set-up costs about 0.06 bands.
+  // Steps on a B200 by waves alone / mean alone / this rule (bands), MP5 HLLC
+  // where not said:
+  //   300 x 300 MC HLL            90.7 (2) / 100.3 (1) / 90.7 us (2)
+  //   512 x 256 MC HLL            150 (3) / 132 (1) / 115 us (2)
+  //   500 x 500 MC HLL            186 (4) / 212 (1) / 195 us (2)
+  //   500 x 500, KH initial data  283 (4) / 325 (1) / 296 us (2)
+  //   900 x 900, KH initial data  869 (13) / 851 (2) / 799 us (3)
+  //   1000 x 500, perturbed       1.19 (8) / 1.08 (2) / 1.08 ms (2)
+  //   2048 x 1024, perturbed      3.87 (10) / 3.73 (3) / 3.74 ms (5)
+  //   4096 x 2048, perturbed      14.19 (13) / 13.95 (5) / 14.00 ms (7)
+  //   24 grids of 128 x 64 to 512 x 256: 3.35 ms by each grid's own waves
+  //   (1, 1 and 3), 3.21 ms (3)
   int best = 1;
-  long long best_cost = -1;
+  double best_cost = 0.0;
   for (int nb = 1; nb <= 32; ++nb) {
     const int seg = nb * rows - 1;
     long long work = 0, longest = 0;   // in bands
@@ -280,8 +290,23 @@ int stage_seg_rows(const int* grids, int ngrids, int rows, int slots) {
       work += (long long)strips * (full * nb + last);
       longest = std::max<long long>(longest, full ? nb : last);
     }
-    const long long cost = 2 * work + slots * longest;
-    if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = nb; }
+    double cost = (double)work / slots + 0.5 * longest;
+    if (ngrids == 1) {
+      const long long strips = stage_tiles(grids[0], 0, seg);
+      const int full = (grids[1] + 1) / seg, rest = (grids[1] + 1) % seg, last = rest ? (rest + rows) / rows : 0;
+      const long long q = strips * full / slots, r = strips * full % slots;   // waves of full tiles, tiles left
+      long long end = (q + (r > 0)) * nb;
+      if (last) {
+        const long long idle = slots - r;
+        long long e = q * nb + (strips + idle - 1) / idle * last;              // all short tiles on the idle slots
+        if (r) e = std::min(e, end + (strips + slots - 1) / slots * last);     // or spread over all
+        end = std::max(end, e);
+      }
+      const bool few = even && stage_tiles(grids[0], grids[1], rows - 1) < 3 * slots;
+      const double w = few ? 0.9 : 0.2;
+      cost = (w * end + (1.0 - w) * cost) * (1.0 + 0.06 / nb);
+    }
+    if (nb == 1 || cost < best_cost) { best_cost = cost; best = nb; }
   }
   return best * rows - 1;
 }

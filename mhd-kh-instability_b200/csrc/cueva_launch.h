@@ -45,8 +45,8 @@ bool stage_fused_available(int rec_mp, int solver);
 int stage_wide_rows(int solver, const int* grids, int ngrids, int num_sms);
 // grid rows per fused-stage tile of a launch over these grids (pairs of imax,
 // jmax): a multiple of rows less one, so that the launch's tiles balance over
-// `slots` resident CTAs
-int stage_seg_rows(const int* grids, int ngrids, int rows, int slots);
+// `slots` resident CTAs; even: bands take like times (the MC routines)
+int stage_seg_rows(const int* grids, int ngrids, int rows, int slots, bool even);
 // pinned host arrays as the kernels see them: element (0, 0) of the 14
 // primitive fields, pitch in doubles
 struct HostPrims {
