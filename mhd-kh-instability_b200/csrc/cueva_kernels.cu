@@ -267,9 +267,9 @@ int stage_seg_rows(const int* grids, int ngrids, int rows, int slots, bool even)
   // with less than three waves of one-band tiles goes by the waves.  A tile's
   // set-up costs about 0.06 bands.
   // Steps on a B200 by waves alone / mean alone / this rule (bands), MP5 HLLC
-  // where not said:
+  // where not said (SSP2 in us, SSP3(4,3,3) in ms):
   //   300 x 300 MC HLL            90.7 (2) / 100.3 (1) / 90.7 us (2)
-  //   512 x 256 MC HLL            150 (3) / 132 (1) / 115 us (2)
+  //   512 x 256 Lax, perturbed    0.300 (3) / 0.279 (1) / 0.249 ms (2)
   //   500 x 500 MC HLL            186 (4) / 212 (1) / 195 us (2)
   //   500 x 500, KH initial data  283 (4) / 325 (1) / 296 us (2)
   //   900 x 900, KH initial data  869 (13) / 851 (2) / 799 us (3)
