@@ -242,7 +242,9 @@ int stage_wide_rows(int solver, const int* grids, int ngrids, int num_sms) {
   // warps a tile: 49), MP7 HLLC 60 (two kernels) / 39; 200 x 100 MP5 44 / 38;
   // 256 x 128 MP5 HLL 42.9 / 40.7, MP9 HLLC 55 / 43.  Where no height up to 12
   // finds an SM for every tile, two CTAs of 8 warps per SM are as good: 320 x
-  // 160 MP5 HLL 45.9 / 45.8 us.
+  // 160 MP5 HLL 45.9 / 45.8 us.  Steps of 15 grids by 10 settings on two flows
+  // gain 0 to 42 %; seen to lose: strips so low that their tiles are few, 500 x 60
+  // MP7 HLLC 163 / 172 us a step (on the other flow 123 / 110), 700 x 40 HLLE 88 / 91.
   if (solver < 5) return 0;
   for (int rows = 4; rows <= WIDE_ROWS; ++rows) {
     long long tiles = 0;

@@ -151,7 +151,7 @@ __device__ __forceinline__ void em_fluxes(const Side<T>& L, const Side<T>& R, T*
 // physical fluxes, so that each pair is folded into its HLL state and flux at
 // once.  With every field reconstructed first, 40 FP64 face values were alive
 // around the last calls of the limiter (128 registers; k_stage HLLC spilled
-// 428 bytes, now 380).  Steps on a B200: 2048 x 4096 HLLC 14.41 -> 14.36 ms,
+// 428 bytes, 380 after).  Steps on a B200: 2048 x 4096 HLLC 14.41 -> 14.36 ms,
 // 700 x 1500 MP9 2.26 -> 2.22 ms, 1024 x 2048 mixed MP7 3.76 -> 3.72 ms.
 
 // PS: split pressure (see physical); A[R_SN] then lacks the reference

@@ -783,7 +783,7 @@ __device__ __forceinline__ uint32_t update_point(const InstDesc& I, const StageA
       // of a zero sum.  The stored K_m (m < l) and this stage's K_l have code
       // of their own: one loop that chose between memory and registers per
       // field kept more of both alive (k_stage MP5 HLLC: 380 bytes of spills,
-      // now 324).  Steps on a B200: 2048 x 4096 14.39 -> 14.10 ms, 1024 x 2048
+      // 324 after).  Steps on a B200: 2048 x 4096 14.39 -> 14.10 ms, 1024 x 2048
       // 3.93 -> 3.85 ms, mixed MP7 3.73 -> 3.69 ms, 611 x 1003 MP7 900 -> 884 us.
       // Loading and storing the sums in two groups of fields instead spilled
       // 490 to 700 bytes: 14.9 to 15.8 ms.

@@ -371,7 +371,7 @@ k_gradients(long long n, int B, unsigned long long seed, long long step, const f
 // it) and, with ADAM, applies the update (Kingma & Ba 2015) and the bf16
 // rounding of the forward copy.  A CTA takes 32 parameters by 8 slices of the
 // rows, each slice in order, the 8 slice sums in order.  B200, 4096 rows,
-// whole gradient call: 600 us before, 57 us with these two kernels (25 + 4 us
+// whole gradient call: 600 us before, 57 us with these two kernels (27 + 5.5 us
 // under ncu, the rest is the copy back); 2000 training steps 1.09 s -> 50 ms.
 template <bool ADAM>
 __global__ void __launch_bounds__(256)
@@ -456,9 +456,11 @@ __global__ void k_c2p_batch(long long n, int method, double gamma, double eps1, 
 // bits.  What bounds it: 8.6 k FMAs per state, 0.23 ms per million states at
 // the FP32 rate.  With one thread per state (mlp_forward) each weight was
 // loaded and widened again for every FMA: 1895 us for 10^6 states on a B200;
-// tiled 622 us; with two states per FMA instruction 600 us (the issue slots
-// go to the recovery's FP64 chains at 12 warps per SM).  mma.sync or tcgen05
-// would round the activations to bf16.
+// tiled 622 us; with two states per FMA instruction 598 us: at 12 warps per SM
+// half of the issue slots are used, by 10.2 k thread instructions a state (6.3 k
+// on the FMA pipe, 0.6 k on the FP64 pipe), the network and the recovery
+// taking turns between barriers.  The bf16 tensor cores would need each FP32
+// activation as three parts; not tried.
 constexpr int CN_ROWS = 128;
 struct C2PNet {
   alignas(16) float w2t[MLP_H * MLP_H], w3t[MLP_H * MLP_H];   // [input][output]
