@@ -276,7 +276,7 @@ int stage_seg_rows(const int* grids, int ngrids, int rows, int slots, bool even)
   //   500 x 500, KH initial data  283 (4) / 325 (1) / 296 us (2)
   //   900 x 900, KH initial data  869 (13) / 851 (2) / 799 us (3)
   //   1000 x 500, perturbed       1.19 (8) / 1.08 (2) / 1.08 ms (2)
-  //   2048 x 1024, perturbed      3.87 (10) / 3.73 (3) / 3.74 ms (5)
+  //   2048 x 1024, perturbed      3.87 (10) / 3.73 (3) / 3.73 ms (3)
   //   4096 x 2048, perturbed      14.19 (13) / 13.95 (5) / 14.00 ms (7)
   //   24 grids of 128 x 64 to 512 x 256: 3.35 ms by each grid's own waves
   //   (1, 1 and 3), 3.21 ms (3)
@@ -305,7 +305,7 @@ int stage_seg_rows(const int* grids, int ngrids, int rows, int slots, bool even)
         end = std::max(end, e);
       }
       const bool few = even && stage_tiles(grids[0], grids[1], rows - 1) < 3 * slots;
-      const double w = few ? 0.9 : 0.2;
+      const double w = few ? 0.9 : 0.1;
       cost = (w * end + (1.0 - w) * cost) * (1.0 + 0.06 / nb);
     }
     if (nb == 1 || cost < best_cost) { best_cost = cost; best = nb; }
