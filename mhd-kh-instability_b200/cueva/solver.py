@@ -120,8 +120,9 @@ class Cueva:
 
     def set_stage_kernel(self, fused):
         """1: one fused kernel per RK stage (the default where it exists: MP5
-        and the MC slopes); 0: the y-face and x-face + update kernels.  Both
-        give bit-identical results."""
+        and the MC slopes; MP7 and MP9 run one on small grids until 0 is set);
+        0: the y-face and x-face + update kernels.  Both give bit-identical
+        results."""
         _abi.check(self.L, self.L.cueva_set_stage_kernel(self.ctx, int(fused)))
 
     def stage_kernel(self):
