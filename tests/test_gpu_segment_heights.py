@@ -2,6 +2,7 @@
 from the grid of its launches: strips of 31 points by segments of 8 nb - 1
 rows, nb being the count measured fastest or within the noise of it."""
 import json
+import time
 
 import pytest
 
@@ -12,7 +13,9 @@ def launched_tiles(path, run):
     """CTAs of each k_stage launch of run()"""
     from torch.profiler import ProfilerActivity, profile
     with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        time.sleep(0.005)   # the launches well inside the recorded window
         run()
+        time.sleep(0.005)
     prof.export_chrome_trace(path)
     with open(path) as f:
         ev = json.load(f)["traceEvents"]
